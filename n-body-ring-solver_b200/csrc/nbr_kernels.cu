@@ -375,9 +375,9 @@ __global__ void __launch_bounds__(WARPS * 32)
 }
 
 // ------------------------------------------------------- FP64 kernel ----
-// The drop-in form: every operation in FP64, the reciprocal square root from
-// CUDA's rsqrt(double).  Matches the reference's double-precision forces up to
-// summation order.  TJ sources per ring stage (x, y, z, m: 32 TJ bytes), UNR
+// The drop-in form: every operation in FP64 (inv_cube; 15 FP64 operations per
+// pair with the 3 differences, 3 for r^2, the mass and 3 sums).  Matches the
+// reference's double-precision forces up to summation order.  TJ sources per ring stage (x, y, z, m: 32 TJ bytes), UNR
 // the unroll depth of the source loop.
 template <int NI, int WARPS, bool EXCL, int TJ, int UNR>
 __global__ void __launch_bounds__(WARPS * 32)
@@ -428,9 +428,7 @@ __global__ void __launch_bounds__(WARPS * 32)
         double r2 = fma(dx, dx, eps2);
         r2 = fma(dy, dy, r2);
         r2 = fma(dz, dz, r2);
-        double y = rsqrt(r2);
-        if (EXCL) y = r2 > 0.0 ? y : 0.0;
-        const double s = mj * (y * y * y);
+        const double s = mj * inv_cube<EXCL>(r2);
         ax[k] = fma(s, dx, ax[k]);
         ay[k] = fma(s, dy, ay[k]);
         az[k] = fma(s, dz, az[k]);
@@ -438,6 +436,10 @@ __global__ void __launch_bounds__(WARPS * 32)
     }
   };
   if (!tile_pipeline(bars, t1 - t0, js, ep.err, issue, body)) return;
+#pragma unroll
+  for (int k = 0; k < NI; ++k) {
+    ax[k] *= kInvCubeScale; ay[k] *= kInvCubeScale; az[k] *= kInvCubeScale;
+  }
   finish<NI>(ip, ep, ibase, lane, xi, yi, zi, ax, ay, az);
 }
 
@@ -565,9 +567,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32)
           double r2 = fma(dx, dx, eps2);
           r2 = fma(dy, dy, r2);
           r2 = fma(dz, dz, r2);
-          double y = rsqrt(r2);
-          if (EXCL) y = r2 > 0.0 ? y : 0.0;
-          const double s = mj * (y * y * y);
+          const double s = mj * inv_cube<EXCL>(r2);
           ax[k] = fma(s, dx, ax[k]);
           ay[k] = fma(s, dy, ay[k]);
           az[k] = fma(s, dz, az[k]);
@@ -587,6 +587,12 @@ __global__ void __launch_bounds__(kSmallWarps * 32)
       ay[2 * p] = (double)h0 + (double)l0; ay[2 * p + 1] = (double)h1 + (double)l1;
       unpack2(hz[p], h0, h1); unpack2(lz[p], l0, l1);
       az[2 * p] = (double)h0 + (double)l0; az[2 * p + 1] = (double)h1 + (double)l1;
+    }
+  }
+  if (PREC == kFP64) {
+#pragma unroll
+    for (int k = 0; k < NI; ++k) {
+      ax[k] *= kInvCubeScale; ay[k] *= kInvCubeScale; az[k] *= kInvCubeScale;
     }
   }
   // Lane groups -> one sum per receiver (every lane of a gl ends with it).
@@ -1138,15 +1144,15 @@ __global__ void __launch_bounds__(kN3F64Warps * 32, 1)
 
 // FP64 form of the Newton-3 kernel (ForceConfig ni = 3 with NBR_FP64): the
 // blocks, CTA map, source rotation and partial-sum layout of k_force_n3_f32c,
-// with every operation in FP64 and the reciprocal square root from CUDA's
-// rsqrt(double), as in k_force_f64; the source tiles are the FP64 x, y, z, m
+// with every operation in FP64; the source tiles are the FP64 x, y, z, m
 // arrays.  Two warps share each row block: warp w of the CTA takes row block
 // a = r0 + w / 2 and, in lane L, its receivers a * kN3Block + 128 (w % 2) +
 // L + 32 q, q < 4 (16 warps, under 128 registers: twice the warps per SM of
-// a one-warp-per-block layout, for the long FP64 rsqrt chain).  Per
-// unordered pair: 3 sub, 3 fma, rsqrt, 2 mul (y^3), 2 mul (m_j y^3, m_i y^3)
-// and 6 fma, against 12 operations and one rsqrt per ordered pair in
-// k_force_f64.  Equal to k_force_f64 up to summation order; deterministic.
+// a one-warp-per-block layout).  Per unordered pair: 3 sub, 3 fma, 5
+// operations of inv_cube, 2 mul (m_j y^3, m_i y^3) and 6 fma = 19, against 15
+// per ordered pair in k_force_f64.  N = 262144 on B200: 1270 GPairs/s with
+// rsqrt(double) and its cube, 1393 with inv_cube.  Equal to k_force_f64 up to
+// summation order; deterministic.
 template <bool EXCL>
 __global__ void __launch_bounds__(kN3F64Warps * 32)
     k_force_n3_f64(const IParticles ip, const JStream js, const N3Params p3, const double eps2,
@@ -1218,9 +1224,7 @@ __global__ void __launch_bounds__(kN3F64Warps * 32)
           double r2 = fma(dx, dx, eps2);
           r2 = fma(dy, dy, r2);
           r2 = fma(dz, dz, r2);
-          double y = rsqrt(r2);
-          if (EXCL) y = r2 > 0.0 ? y : 0.0;
-          const double s = mj * (y * y * y);
+          const double s = mj * inv_cube<EXCL>(r2);
           AX[q] = fma(s, dx, AX[q]);
           AY[q] = fma(s, dy, AY[q]);
           AZ[q] = fma(s, dz, AZ[q]);
@@ -1244,9 +1248,7 @@ __global__ void __launch_bounds__(kN3F64Warps * 32)
             double r2 = fma(dx, dx, eps2);
             r2 = fma(dy, dy, r2);
             r2 = fma(dz, dz, r2);
-            double y = rsqrt(r2);
-            if (EXCL) y = r2 > 0.0 ? y : 0.0;
-            const double y3 = y * y * y;
+            const double y3 = inv_cube<EXCL>(r2);
             const double sj = ms * y3, si = mi[q] * y3;
             // reaction first, and its shuffles before the sources': the faster
             // schedule (+1.7 % at N = 262144), as in k_force_n3_f32c
@@ -1287,6 +1289,7 @@ __global__ void __launch_bounds__(kN3F64Warps * 32)
         for (int d = 0; d < 3; ++d) {
           double s = 0.0;
           for (int w = 0; w < kN3F64Warps; ++w) s += red[(w * 3 + d) * kN3Block + tid];
+          s *= kInvCubeScale;
           if (NBR_IN((p3.rea - p3.act) + off + d * kN3Block + tid, p3.act_len, err))
             out[d * kN3Block + tid] = s;
         }
@@ -1300,9 +1303,9 @@ __global__ void __launch_bounds__(kN3F64Warps * 32)
     return;
 #pragma unroll
   for (int q = 0; q < NI; ++q) {
-    act[lane + 32 * q] = AX[q];
-    act[kN3Block + lane + 32 * q] = AY[q];
-    act[2 * kN3Block + lane + 32 * q] = AZ[q];
+    act[lane + 32 * q] = kInvCubeScale * AX[q];
+    act[kN3Block + lane + 32 * q] = kInvCubeScale * AY[q];
+    act[2 * kN3Block + lane + 32 * q] = kInvCubeScale * AZ[q];
   }
 }
 

@@ -23,8 +23,7 @@
 // for the host, if the limit passes or another CTA has already recorded an
 // error.  The cooperative launch guarantees that all CTAs are resident, so no
 // CTA waits on one that cannot run.  FP64 pair arithmetic is k_force_f64's
-// (CUDA's rsqrt(double)): results equal the other FP64 kernels' up to
-// summation order; the FP32C form (k_run_small_f32c) is described there.
+// (inv_cube): results equal the other FP64 kernels' up to summation order; the FP32C form (k_run_small_f32c) is described there.
 #include "nbr.h"
 #include "nbr_ctx.h"
 #include "nbr_device.cuh"
@@ -211,9 +210,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_run_small_f64(const PersistArgs A
           double r2 = fma(dx, dx, A.eps2);
           r2 = fma(dy, dy, r2);
           r2 = fma(dz, dz, r2);
-          double y = rsqrt(r2);
-          if (EXCL) y = r2 > 0.0 ? y : 0.0;
-          const double s = mj * (y * y * y);
+          const double s = mj * inv_cube<EXCL>(r2);
           ax[k] = fma(s, dx, ax[k]);
           ay[k] = fma(s, dy, ay[k]);
           az[k] = fma(s, dz, az[k]);
@@ -245,6 +242,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_run_small_f64(const PersistArgs A
           const double* r = red + ((size_t)w * RPC + t) * 3;
           a0 += r[0]; a1 += r[1]; a2 += r[2];
         }
+        a0 *= kInvCubeScale; a1 *= kInvCubeScale; a2 *= kInvCubeScale;
         if (t < A.cs && i < n) {
           // the epilogue of the large kernels: a -> acc, v += kick a, x' = x + drift v
           // (Euler: drift with the old velocity)
