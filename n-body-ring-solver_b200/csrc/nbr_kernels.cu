@@ -925,10 +925,10 @@ __global__ void __launch_bounds__(kN3Warps * 32)
 // reaction staging sums the two warps' halves in warp order; the results
 // equal k_force_n3_f32c's to FP32 rounding of the per-warp reaction sums.
 template <bool EXCL>
-__global__ void __launch_bounds__(kN3F64Warps * 32, 1)
+__global__ void __launch_bounds__(kN3W2Warps * 32, 1)
     k_force_n3_f32c_w2(const IParticles ip, const JStream js, const N3Params p3, const float eps2f,
                        int* err) {
-  constexpr int NI = 4, IPAIR = 2, WARPS = kN3F64Warps;
+  constexpr int NI = 4, IPAIR = 2, WARPS = kN3W2Warps;
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
   unsigned char* stages = smem + kSmemHead;
@@ -1143,27 +1143,33 @@ __global__ void __launch_bounds__(kN3F64Warps * 32, 1)
 }
 
 // FP64 form of the Newton-3 kernel (ForceConfig ni = 3 with NBR_FP64): the
-// blocks, CTA map, source rotation and partial-sum layout of k_force_n3_f32c,
-// with every operation in FP64; the source tiles are the FP64 x, y, z, m
-// arrays.  Two warps share each row block: warp w of the CTA takes row block
-// a = r0 + w / 2 and, in lane L, its receivers a * kN3Block + 128 (w % 2) +
-// L + 32 q, q < 4 (16 warps, under 128 registers: twice the warps per SM of
-// a one-warp-per-block layout).  Per unordered pair: 3 sub, 3 fma, 5
-// operations of inv_cube, 2 mul (m_j y^3, m_i y^3) and 6 fma = 19, against 15
-// per ordered pair in k_force_f64.  N = 262144 on B200: 1270 GPairs/s with
-// rsqrt(double) and its cube, 1393 with inv_cube.  Equal to k_force_f64 up to
-// summation order; deterministic.
+// blocks, CTA map and partial-sum layout of k_force_n3_f32c, with every
+// operation in FP64; the source tiles are the FP64 x, y, z, m arrays.  One
+// warp per row block, 8 receivers per lane.  Per unordered pair: 3 sub, 3 fma,
+// 5 operations of inv_cube, 2 mul (m_j y^3, m_i y^3) and 6 fma = 19, against
+// 15 per ordered pair in k_force_f64.
+//
+// What bounds it: the register-file ports of the FP64 pipe.  An fma whose
+// three operands are distinct registers issues at 47.9 lanes per clock and SM,
+// one that shares an operand with its neighbour at 54.7, an add at 63.9
+// (measured), so the loop reaches about 53 of 64.  Rotating a source and its
+// reaction by shuffles costs 14 per step, whatever the receivers: 8 receivers
+// per lane halve that per pair, and the sources are read from the tile in
+// shared memory instead (lane l takes source (l + step) mod 32, one step
+// ahead), so only the three reaction sums rotate.  N = 262144, GPairs/s: 1393
+// with two warps of 4 receivers per row block and shuffled sources, 1517 with
+// 8 receivers, 1556 with the sources from shared memory.  Equal to
+// k_force_f64 up to summation order; deterministic.
 template <bool EXCL>
-__global__ void __launch_bounds__(kN3F64Warps * 32)
+__global__ void __launch_bounds__(kN3F64Warps * 32, 1)
     k_force_n3_f64(const IParticles ip, const JStream js, const N3Params p3, const double eps2,
                    int* err) {
-  constexpr int NI = kN3Block / 64;
+  constexpr int NI = kN3Block / 32;
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
   unsigned char* stages = smem + kSmemHead;
   double* red = reinterpret_cast<double*>(stages + kStages * kStage64);  // [warp][3][256]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int rb = warp >> 1, hf = warp & 1;  // row block in the group, its receiver half
   int g = p3.g0, k = p3.order ? p3.order[blockIdx.x] : (int)blockIdx.x;  // group-major number
   const int groups = p3.g1;  // row groups [g0, g1) of this launch
   while (g < groups) {  // the grid has exactly sum_g n3_chunks(nb, cols, g) CTAs
@@ -1174,12 +1180,12 @@ __global__ void __launch_bounds__(kN3F64Warps * 32)
   }
   if (g >= groups) return;
   const long long r0 = (long long)g * kN3Warps;
-  const long long a = r0 + rb;
+  const long long a = r0 + warp;
   const long long cs = r0 + (long long)k * p3.cols;
   const long long ce = min(cs + (long long)p3.cols, p3.nb);
   const int ntl = (int)(2 * (ce - cs));
   const bool row_ok = a < p3.nb;
-  const long long ibase = a * kN3Block + hf * (kN3Block / 2) + lane;
+  const long long ibase = a * kN3Block + lane;
 
   double xi[NI], yi[NI], zi[NI], mi[NI], AX[NI], AY[NI], AZ[NI];
 #pragma unroll
@@ -1234,14 +1240,16 @@ __global__ void __launch_bounds__(kN3F64Warps * 32)
       for (int bt = 0; bt < 4; ++bt)
         myred[bt * 32 + lane] = myred[kN3Block + bt * 32 + lane] = myred[2 * kN3Block + bt * 32 + lane] = 0.0;
     } else if (row_ok && c > a) {
-      const int from = (lane + 31) & 31;
+      const int from = (lane + 1) & 31;
 #pragma unroll 1
       for (int bt = 0; bt < 4; ++bt) {
-        const int j = bt * 32 + lane;
-        double xs = sx[j], ys = sy[j], zs = sz[j], ms = sm[j];
+        const double *bx = sx + bt * 32, *by = sy + bt * 32, *bz = sz + bt * 32, *bm = sm + bt * 32;
+        double xs = bx[lane], ys = by[lane], zs = bz[lane], ms = bm[lane];
         double RX = 0.0, RY = 0.0, RZ = 0.0;
-#pragma unroll 1  // 3 % faster than unrolled by 2 or 4 (N = 262144)
+#pragma unroll 2
         for (int step = 0; step < 32; ++step) {
+          const int jn = (lane + step + 1) & 31;  // the next step's source
+          const double xn = bx[jn], yn = by[jn], zn = bz[jn], mn = bm[jn];
 #pragma unroll
           for (int q = 0; q < NI; ++q) {
             const double dx = xs - xi[q], dy = ys - yi[q], dz = zs - zi[q];
@@ -1250,8 +1258,6 @@ __global__ void __launch_bounds__(kN3F64Warps * 32)
             r2 = fma(dz, dz, r2);
             const double y3 = inv_cube<EXCL>(r2);
             const double sj = ms * y3, si = mi[q] * y3;
-            // reaction first, and its shuffles before the sources': the faster
-            // schedule (+1.7 % at N = 262144), as in k_force_n3_f32c
             RX = fma(si, dx, RX);
             RY = fma(si, dy, RY);
             RZ = fma(si, dz, RZ);
@@ -1262,10 +1268,7 @@ __global__ void __launch_bounds__(kN3F64Warps * 32)
           RX = __shfl_sync(0xffffffffu, RX, from);
           RY = __shfl_sync(0xffffffffu, RY, from);
           RZ = __shfl_sync(0xffffffffu, RZ, from);
-          xs = __shfl_sync(0xffffffffu, xs, from);
-          ys = __shfl_sync(0xffffffffu, ys, from);
-          zs = __shfl_sync(0xffffffffu, zs, from);
-          ms = __shfl_sync(0xffffffffu, ms, from);
+          xs = xn; ys = yn; zs = zn; ms = mn;
         }
         // back at its own lane: the force on source j is -sum m_i y^3 d
         myred[bt * 32 + lane] = -RX;
@@ -1298,8 +1301,8 @@ __global__ void __launch_bounds__(kN3F64Warps * 32)
     }
   };
   if (!tile_pipeline(bars, ntl, js, err, issue, body)) return;
-  double* act = p3.act + ((size_t)blockIdx.x * kN3Warps + rb) * 3 * kN3Block + hf * (kN3Block / 2);
-  if (!NBR_IN(((long long)blockIdx.x * kN3Warps + rb + 1) * 3 * kN3Block - 1, p3.act_len, err))
+  double* act = p3.act + ((size_t)blockIdx.x * kN3Warps + warp) * 3 * kN3Block;
+  if (!NBR_IN(((long long)blockIdx.x * kN3Warps + warp + 1) * 3 * kN3Block - 1, p3.act_len, err))
     return;
 #pragma unroll
   for (int q = 0; q < NI; ++q) {
@@ -1721,6 +1724,10 @@ cudaError_t launch_small_t(double eps2, int split, const IParticles& ip, const J
 
 }  // namespace
 
+// Warps per CTA of the Newton-3 kernel for a configuration's `warps`.
+static int n3_cta_warps(int precision, int warps) {
+  return precision == kFP64 ? kN3F64Warps : warps == kN3W2Warps ? kN3W2Warps : kN3Warps;
+}
 size_t n3_smem_bytes(int precision, int warps);
 
 bool force_config_supported(int precision, const ForceConfig& c) {
@@ -1731,8 +1738,8 @@ bool force_config_supported(int precision, const ForceConfig& c) {
     return (c.split <= 1 || c.split == 8 || c.split == 16) &&
            (((c.tile == 0 || c.tile == 4) && f4) || (c.tile == 8 && (c.warps == 8 || c.warps == 16)));
   }
-  if (c.ni == 3)  // Newton-3: FP32C one or two warps per row block; FP64 (two)
-    return c.warps == kN3Warps || (precision == kFP32C && c.warps == kN3F64Warps);
+  if (c.ni == 3)  // Newton-3: FP32C one or two warps per row block; FP64 one
+    return c.warps == kN3Warps || (precision == kFP32C && c.warps == kN3W2Warps);
   if (c.ni == 1) return (c.warps == 2 || c.warps == 4 || c.warps == 8) && c.split >= 1;
   if (c.split < 1) return false;
   return large_fn(precision, c.ni, c.warps, norm_tile(c), norm_unroll(precision, c), false) != nullptr;
@@ -1742,12 +1749,12 @@ int force_blocks_per_sm(int precision, double eps2, const ForceConfig& c) {
   int nb = 0;
   if (c.ni == 3) {
     const bool ex = eps2 == 0.0;
-    const bool w2 = precision == kFP32C && c.warps == kN3F64Warps;
+    const bool w2 = precision == kFP32C && c.warps == kN3W2Warps;
     const void* fn = precision == kFP32C
                          ? (w2 ? (ex ? (const void*)k_force_n3_f32c_w2<true> : (const void*)k_force_n3_f32c_w2<false>)
                                : (ex ? (const void*)k_force_n3_f32c<true, false> : (const void*)k_force_n3_f32c<false, false>))
                          : (ex ? (const void*)k_force_n3_f64<true> : (const void*)k_force_n3_f64<false>);
-    const int threads = (precision == kFP32C && !w2 ? kN3Warps : kN3F64Warps) * 32;
+    const int threads = n3_cta_warps(precision, c.warps) * 32;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, threads, n3_smem_bytes(precision, c.warps)) !=
         cudaSuccess)
       nb = 0;
@@ -1985,7 +1992,7 @@ cudaError_t configure_kernels() {
   // The Newton-3 kernels need more than the default 48 KB of dynamic shared
   // memory; set once per device, outside any stream capture.
   const int s32 = (int)n3_smem_bytes(kFP32C, kN3Warps), s64 = (int)n3_smem_bytes(kFP64, kN3F64Warps);
-  const int s32w = (int)n3_smem_bytes(kFP32C, kN3F64Warps);
+  const int s32w = (int)n3_smem_bytes(kFP32C, kN3W2Warps);
   const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
   cudaError_t e = cudaFuncSetAttribute((const void*)k_force_n3_f32c<true, false>, at, s32);
   if (e == cudaSuccess) e = cudaFuncSetAttribute((const void*)k_force_n3_f32c<false, false>, at, s32);
@@ -2024,10 +2031,9 @@ cudaError_t launch_force_n3(int precision, int warps, double eps2, const IPartic
   p3.order = order;
   p3.slot = order ? order + ctas : nullptr;
   NBR_CHECKED_ONLY(p3.act_len = scratch_len;)
-  const bool w2 = precision == kFP32C && warps == kN3F64Warps;
-  const size_t smem = n3_smem_bytes(precision, precision == kFP32C ? warps : kN3F64Warps);
-  const unsigned grid = (unsigned)ctas,
-                 block = (precision == kFP32C && !w2 ? kN3Warps : kN3F64Warps) * 32;
+  const bool w2 = precision == kFP32C && warps == kN3W2Warps;
+  const size_t smem = n3_smem_bytes(precision, warps);
+  const unsigned grid = (unsigned)ctas, block = n3_cta_warps(precision, warps) * 32;
   if (w2) {
     if (eps2 == 0.0)
       k_force_n3_f32c_w2<true><<<grid, block, smem, st>>>(ip, js, p3, 0.f, ep.err);
@@ -2063,10 +2069,9 @@ cudaError_t launch_n3_pairs(int precision, int warps, double eps2, const IPartic
   const long long ctas = n3_ctas_range(p3.nb, p3.cols, p3.g0, p3.g1);
   if (ctas <= 0) return cudaSuccess;
   if (ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  const bool w2 = precision == kFP32C && warps == kN3F64Warps;
-  const size_t smem = n3_smem_bytes(precision, precision == kFP32C ? warps : kN3F64Warps);
-  const unsigned grid = (unsigned)ctas,
-                 block = (precision == kFP32C && !w2 ? kN3Warps : kN3F64Warps) * 32;
+  const bool w2 = precision == kFP32C && warps == kN3W2Warps;
+  const size_t smem = n3_smem_bytes(precision, warps);
+  const unsigned grid = (unsigned)ctas, block = n3_cta_warps(precision, warps) * 32;
   const float e32 = (float)eps2;
   if (w2) {
     if (eps2 == 0.0) k_force_n3_f32c_w2<true><<<grid, block, smem, st>>>(ip, js, p3, 0.f, err);

@@ -94,7 +94,8 @@ constexpr int kSmallNI = 4;
 // particles, kN3Warps row blocks per CTA (one per warp), up to `cols` column
 // blocks per CTA (n3_cols, n3_slice_cols: at most kN3MaxCols).
 constexpr int kN3Warps = 8;
-constexpr int kN3F64Warps = 2 * kN3Warps;  // FP64: two warps per row block
+constexpr int kN3F64Warps = kN3Warps;     // FP64: one warp per row block
+constexpr int kN3W2Warps = 2 * kN3Warps;  // FP32C form with two warps per row block
 constexpr int kN3Block = 256;
 constexpr int kN3MaxCols = 32;
 struct N3Params {
@@ -205,7 +206,7 @@ inline long long n3_slice_scratch_doubles(long long nb, int v, int V) {
 // with the epilogue ep: the pair kernel, then the per-particle reduction.
 // scratch holds n3_scratch_doubles(ceil(n / kN3Block)) doubles; order is the
 // grid's launch order (n3_launch_order, on the device).
-// FP32C: warps = kN3Warps (one warp per row block) or kN3F64Warps (two).
+// FP32C: warps = kN3Warps (one warp per row block) or kN3W2Warps (two).
 cudaError_t launch_force_n3(int precision, int warps, double eps2, const IParticles& ip,
                             const JStream& js, const Epilogue& ep, double* scratch,
                             long long scratch_len, const int* order, cudaStream_t stream);
