@@ -308,7 +308,10 @@ int auto_split(int precision, double eps2, const ForceConfig& c, long long n_i, 
   return (int)s;
 }
 
-ForceConfig choose_config(nbr_ctx* c, int precision, double eps2, long long n_i, int ntiles) {
+// whole: an evaluation of the whole system, which the Newton-3 strips can
+// take; receiver ranges and separate receiver and source sets cannot.
+ForceConfig choose_config(nbr_ctx* c, int precision, double eps2, long long n_i, int ntiles,
+                          bool whole = true) {
   ForceConfig cfg = c->override_cfg[precision];
   if (cfg.ni == kPersistNI) cfg = ForceConfig{0, 0, 0};  // a run-level choice: evaluations use the default
   if (cfg.ni == 0) {
@@ -325,18 +328,11 @@ ForceConfig choose_config(nbr_ctx* c, int precision, double eps2, long long n_i,
     // that the large kernels win.
     const int F = precision == kFP32C ? (n_i <= 4096 ? 8 : n_i <= 8192 ? 2 : 0)
                                       : (n_i <= 16384 ? 8 : n_i <= 32768 ? 4 : 0);
-    // From 16384 to 2^20 particles: the Newton-3 kernels (B200, against the
-    // best other kernel: FP32C +24 % at N = 262144 and +28 % at 2^20; FP64
-    // +16 % at 16384, +20 % at 32768, +30 % at 262144, +33 % at 2^20).
-    if (n_i >= kN3MinN && n_i <= kN3MaxN) dflt = ForceConfig{3, kN3Warps, 0};
-    // From 8192 up: the Newton-3 kernels where the grid model gives them a good
-    // last wave.  Their advantage followed the modeled grid efficiency on B200
-    // (N = 8192 .. 15360 in steps of 1024): efficiency >= 0.70, FP32C +28 to
-    // +31 % and FP64 +12 to +17 %; 0.60 - 0.63, FP32C +6 to +11 %, FP64 -0.2 to
-    // +3 %; <= 0.55, a loss.
-    else if (n_i >= 8192 &&
-             n3_grid_efficiency((n_i + kN3Block - 1) / kN3Block) >= (precision == kFP32C ? 0.60 : 0.65))
-      dflt = ForceConfig{3, kN3Warps, 0};
+    // From there to 2^23 particles: Newton-3 (B200, us per KDK step, the best
+    // kernel above against the strips: FP32C 4608 33.6 / 17.8, 6000 42.6 / 22.4,
+    // 8192 53.6 / 33.4, 12001 108.6 / 61.9; FP64 36.7 / 27.9, 56.1 / 34.7, 87.8 /
+    // 57.3, 164 / 114; and larger systems, see uses_strips and nbr_strip.cu).
+    if (whole && n_i >= kN3MinN && n_i <= kN3MaxN) dflt = ForceConfig{3, kN3Warps, 0};
     else if (F) dflt = ForceConfig{1, F, 0};
     cfg = it != g_tune->end() ? it->second : dflt;
   }
@@ -356,16 +352,19 @@ ForceConfig choose_config_large(nbr_ctx* c, int precision, double eps2, long lon
   return cfg;
 }
 
-// Prepares scratch for a force launch of `cfg` over n_i receivers.
-// Slices of a banded Newton-3 evaluation of nb blocks (1: one launch).
-// Test hook: NBR_TEST_N3_SLICES=k forces k slices on any system, so that the
-// banded path (slice partials accumulated in order, then the epilogue) runs
-// on systems small enough to check against the oracle.
+// Test hook: NBR_TEST_N3_SLICES=k forces k launches of a Newton-3 evaluation on
+// any system, so that the banded path (partial sums accumulated launch by
+// launch, then the epilogue) runs on systems small enough to check against
+// the oracle.  0: not set.
+int forced_bands() {
+  const char* f = std::getenv("NBR_TEST_N3_SLICES");
+  return f ? std::max(0, std::atoi(f)) : 0;
+}
+
+// Slices of a banded evaluation of nb blocks by the CTA-grid kernel (1: one
+// launch).
 int n3_bands(long long nb) {
-  if (const char* f = std::getenv("NBR_TEST_N3_SLICES")) {
-    const int k = std::atoi(f);
-    if (k >= 1) return k;
-  }
+  if (const int k = forced_bands()) return k;
   const long long total = n3_scratch_doubles(nb);
   if (total <= kN3SingleMaxDoubles) return 1;
   int V = (int)((total + kN3SliceMaxDoubles - 1) / kN3SliceMaxDoubles);
@@ -415,7 +414,43 @@ cudaError_t n3_order_prepare(nbr_ctx* c, long long nb) {
   return e;
 }
 
-int prepare_split(nbr_ctx* c, const ForceConfig& cfg, long long n_pad_i) {
+// The launches of a Newton-3 evaluation of the context's system in strips:
+// receivers per lane, the row blocks at which they begin and end, and the
+// scratch: the largest launch's partial sums, then, where there are several
+// launches, the FP64 accumulator [3][n_pad].
+struct StripLaunches {
+  int ni = 0;
+  std::vector<int> cut;
+  long long acc_off = 0, doubles = 0;
+};
+StripLaunches strip_launches(nbr_ctx* c, int precision) {
+  StripLaunches L;
+  const long long n = (long long)c->sys.n;
+  L.ni = strip_choose(precision, n, c->sms);
+  L.cut = strip_bands(precision, n, c->sms, L.ni, forced_bands());
+  for (size_t v = 0; v + 1 < L.cut.size(); ++v)
+    L.doubles = std::max(
+        L.doubles, strip_plan(precision, n, L.cut[v], L.cut[v + 1], c->sms, L.ni).doubles);
+  if (L.cut.size() > 2) {
+    L.acc_off = (L.doubles + 31) / 32 * 32;
+    L.doubles = L.acc_off + 3 * (long long)c->sys.n_pad;
+  }
+  return L;
+}
+// FP32C: every whole system.  FP64: up to kStripMaxN64 particles (us per
+// evaluation on B200, CTA grid against strips: 32768 812 / 722, 65536 2904 /
+// 2840, 131072 11323 / 11293, 262144 44156 / 44625, 2^20 705 / 718 ms: the
+// strips' 24 B of reactions per (320 rows, particle) take more launches).
+bool uses_strips(int precision, const ForceConfig& cfg, long long n) {
+  return cfg.ni == 3 && cfg.warps == kN3Warps && (precision == kFP32C || n <= kStripMaxN64);
+}
+
+// Prepares scratch for a force launch of `cfg` over n_i receivers.
+int prepare_split(nbr_ctx* c, int precision, const ForceConfig& cfg, long long n_pad_i) {
+  if (uses_strips(precision, cfg, (long long)c->sys.n)) {  // (the context's whole system only)
+    const cudaError_t e = c->scr.need_part((size_t)strip_launches(c, precision).doubles);
+    return e == cudaSuccess ? NBR_OK : cuda_fail(c, e, "Newton-3 scratch");
+  }
   if (cfg.ni == 3) {  // Newton-3 (the context's whole system only): its own partial sums
     (void)n_pad_i;
     const long long nb = ((long long)c->sys.n + kN3Block - 1) / kN3Block;
@@ -499,12 +534,13 @@ int eval_system(nbr_ctx* c, int precision, double G, double eps2, int mode, doub
   }
   const long long np_i = ((rn + 1023) / 1024) * 1024;
   cudaError_t e = cudaSuccess;
-  if (precision == kFP32C) e = ensure_records(c, a, kernels);
-  if (e != cudaSuccess) return cuda_fail(c, e, "pack");
-  ForceConfig cfg = choose_config(c, precision, eps2, rn, s.ntiles);
+  ForceConfig cfg = choose_config(c, precision, eps2, rn, s.ntiles, !ranged);
   if (cfg.ni == 3 && ranged)  // needs the whole system
     cfg = choose_config_large(c, precision, eps2, rn, s.ntiles);
-  int rc = prepare_split(c, cfg, np_i);
+  const bool strips = uses_strips(precision, cfg, rn);  // these read the FP64 positions: no records
+  if (precision == kFP32C && !strips) e = ensure_records(c, a, kernels);
+  if (e != cudaSuccess) return cuda_fail(c, e, "pack");
+  int rc = prepare_split(c, precision, cfg, np_i);
   if (rc) return rc;
   IParticles ip{s.pos[a][0] + r0, s.pos[a][1] + r0, s.pos[a][2] + r0, s.mass + r0, rn};
   JStream js{s.pos[a][0], s.pos[a][1], s.pos[a][2], s.mass, s.rec[a], s.org[a], s.ntiles, 0, -1};
@@ -518,8 +554,9 @@ int eval_system(nbr_ctx* c, int precision, double G, double eps2, int mode, doub
   ep.drift = drift;
   ep.vx = s.vel[0] + r0; ep.vy = s.vel[1] + r0; ep.vz = s.vel[2] + r0;
   ep.xn = s.pos[b][0] + r0; ep.yn = s.pos[b][1] + r0; ep.zn = s.pos[b][2] + r0;
-  const bool small = cfg.ni == 1;  // the small-N kernel packs no records
-  ep.rec_next = (mode != 0 && precision == kFP32C && !ranged && !small) ? s.rec[b] : nullptr;
+  // neither the small-N kernel nor the strips pack records
+  const bool packs = precision == kFP32C && !ranged && cfg.ni != 1 && !strips;
+  ep.rec_next = mode != 0 && packs ? s.rec[b] : nullptr;
   ep.origin_next = s.org[b];
   ep.part = c->scr.part;
   ep.counters = c->scr.cnt;
@@ -531,7 +568,22 @@ int eval_system(nbr_ctx* c, int precision, double G, double eps2, int mode, doub
       ep.rec_len = (long long)s.cap;
       // test hook: under-report the receivers' length so that the check trips
       if (std::getenv("NBR_TEST_SHRINK_BOUNDS")) ip.len = rn - 1;)
-  if (cfg.ni == 3) {
+  if (strips) {
+    const StripLaunches L = strip_launches(c, precision);
+    const bool one = L.cut.size() == 2;
+    const long long np = (long long)s.n_pad;
+    double* acc = c->scr.part + L.acc_off;
+    for (size_t v = 0; v + 1 < L.cut.size() && e == cudaSuccess; ++v) {
+      const StripPlan sp = strip_plan(precision, rn, L.cut[v], L.cut[v + 1], c->sms, L.ni);
+      e = launch_strips(precision, sp, eps2, ip, js, ep, c->scr.part, c->sms,
+                        one ? 0 : v == 0 ? 1 : 2, acc, np, c->stream);
+      if (kernels) *kernels += 2;
+    }
+    if (!one) {
+      if (e == cudaSuccess) e = launch_sum_finish(ip, ep, acc, 1, 0, np, 3 * np, c->stream);
+      if (kernels) *kernels += 1;
+    }
+  } else if (cfg.ni == 3) {
     const long long nb = (rn + kN3Block - 1) / kN3Block;
     const int V = n3_bands(nb);
     if (V == 1) {
@@ -560,7 +612,7 @@ int eval_system(nbr_ctx* c, int precision, double G, double eps2, int mode, doub
   if (e != cudaSuccess) return cuda_fail(c, e, "force launch");
   if (mode != 0) {
     s.cur = b;
-    s.rec_ok[b] = (precision == kFP32C) && !ranged && !small;
+    s.rec_ok[b] = packs;
     s.rec_ok[a] = false;
   }
   return NBR_OK;
@@ -595,7 +647,7 @@ int potential_system(nbr_ctx* c, double G, double eps2, double* dphi, size_t red
   int split = auto_split(kFP64, eps2, pc, (long long)s.n, s.ntiles, c->sms);
   split = std::max(1, std::min(split, s.ntiles));
   const ForceConfig cfg{kPotNI, kPotWarps, split};
-  int rc = prepare_split(c, cfg, (long long)s.n_pad);
+  int rc = prepare_split(c, kFP64, cfg, (long long)s.n_pad);
   if (rc) return rc;
   const long long chunk = 32LL * kPotNI * kPotWarps;
   const int chunks = (int)(((long long)s.n + chunk - 1) / chunk);
@@ -732,6 +784,7 @@ int nbr_ctx_create(int device, nbr_ctx** out) {
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
   if (e == cudaSuccess) e = dalloc((void**)&c->d_err, sizeof(int) * 4);
   if (e == cudaSuccess) e = configure_kernels();
+  if (e == cudaSuccess) e = configure_strips();
   if (e != cudaSuccess) {
     int rc = cuda_fail(nullptr, e, "context setup");
     nbr_ctx_destroy(c);
@@ -1099,9 +1152,9 @@ int nbr_accel_ij(nbr_ctx* c, int precision, size_t n_i, const double* xi, const 
                           nullptr, nullptr, r.rec[1], r.org[1], c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "ij pack");
   }
-  ForceConfig cfg = choose_config(c, precision, eps2, (long long)n_i, ntiles);
+  ForceConfig cfg = choose_config(c, precision, eps2, (long long)n_i, ntiles, false);
   if (cfg.ni == 3) cfg = choose_config_large(c, precision, eps2, (long long)n_i, ntiles);
-  int rc = prepare_split(c, cfg, npi);
+  int rc = prepare_split(c, precision, cfg, npi);
   if (rc) return rc;
   IParticles ip{r.pos[0][0], r.pos[0][1], r.pos[0][2], r.mass, (long long)n_i};
   // (the source masses are staged in r.vel[0])
@@ -1209,7 +1262,7 @@ int nbr_run(nbr_ctx* c, int precision, int scheme, int order, double dt, size_t 
   } else if (steps > 0) {
     // Allocate everything the sequence needs before capture.
     ForceConfig cfg = choose_config(c, precision, eps2, (long long)s.n, s.ntiles);
-    rc = prepare_split(c, cfg, (long long)s.n_pad);
+    rc = prepare_split(c, precision, cfg, (long long)s.n_pad);
     if (rc) return rc;
     const bool fsal = (scheme == NBR_KDK) && c->acc_ok && c->acc_prec == precision &&
                       c->acc_G == G && c->acc_eps2 == eps2;
@@ -1248,7 +1301,7 @@ int nbr_run(nbr_ctx* c, int precision, int scheme, int order, double dt, size_t 
       const int cur0 = s.cur;
       const bool rec0 = s.rec_ok[0], rec1 = s.rec_ok[1];
       rc = NBR_OK;
-      const bool fp32 = precision == kFP32C;
+      const bool fp32 = precision == kFP32C && !uses_strips(precision, cfg, (long long)s.n);
       if (scheme == NBR_KDK) {
         if (fsal) {
           rc = kick_drift_system(c, fp32, 0.5 * dt, dt, true, &kernels);

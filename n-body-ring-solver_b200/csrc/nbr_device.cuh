@@ -59,6 +59,10 @@ __device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
   return d;
 }
+// c - a b (the sign of a flipped off the FMA pipe).
+__device__ __forceinline__ u64 fnma2(u64 a, u64 b, u64 c) {
+  return fma2(a ^ 0x8000000080000000ull, b, c);
+}
 // MUFU reciprocal square root of each half.
 __device__ __forceinline__ float rsqrt_mufu(float x) {
   float y;

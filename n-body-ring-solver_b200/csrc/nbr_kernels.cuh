@@ -122,8 +122,9 @@ constexpr long long kN3SingleMaxDoubles = 9LL << 27;  // 9 GiB
 constexpr long long kN3SliceMaxDoubles = 1LL << 28;   // 2 GiB
 // Largest system the Newton-3 kernel is the default for.
 constexpr long long kN3MaxN = 1LL << 23;
-// Smallest system the default configuration gives the Newton-3 kernel.
-constexpr long long kN3MinN = 16384;
+// Smallest system the default configuration evaluates by Newton-3 strips
+// (smaller ones: the small-N kernel, and for nbr_run one persistent launch).
+constexpr long long kN3MinN = 4097;
 // Column chunks (CTAs) of row group g.
 __host__ __device__ inline int n3_chunks(long long nb, int cols, int g) {
   const long long left = nb - (long long)g * kN3Warps;
@@ -230,6 +231,38 @@ cudaError_t launch_n3_slices(int precision, int warps, double eps2, const IParti
 cudaError_t launch_sum_finish(const IParticles& ip, const Epilogue& ep, const double* src, int V,
                               long long vstride, long long ld, long long src_len,
                               cudaStream_t stream);
+// The Newton-3 evaluation in strips (nbr_strip.cu), the default for whole
+// systems above kPersistMaxN particles: one warp per strip of (row block of
+// 32 tb receivers, batch of 32 sources) units, kStripWarps warps per CTA, one
+// CTA per SM.
+constexpr int kStripWarps = 8;
+constexpr long long kStripMaxN64 = 3LL << 16;  // FP64: the CTA grid above
+struct StripPlan {
+  int batches;            // batches of 32 sources
+  int rows;               // row blocks of the system
+  int r0, r1;             // row blocks of this launch
+  int tb;                 // receivers per lane = own batches of a row block
+  int units;              // units of this launch
+  int strips;             // warps that hold a strip
+  int share, longer;      // units per strip; the first `longer` strips hold one more
+  long long act_doubles;  // action partial sums
+  long long reactions;    // reaction partial sums (floats for FP32C, doubles for FP64)
+  long long doubles;      // scratch: the actions, then the reactions
+};
+// The plan of row blocks [r0, min(r1, rows)), ni = tb receivers per lane.
+StripPlan strip_plan(int precision, long long n, int r0, int r1, int sms, int ni);
+// Receivers per lane for a whole system.
+int strip_choose(int precision, long long n, int sms);
+// The row blocks at which an evaluation's launches begin and, last, their count.
+std::vector<int> strip_bands(int precision, long long n, int sms, int ni, int bands);
+// The strips of plan p over the FP64 particles of js (the receivers ip are the
+// same particles), then the reduction: mode 0 runs the epilogue ep (which
+// writes no FP32C records), 1 stores the accelerations over G of all particles
+// into dst[d * ld + i], 2 adds them to it.
+cudaError_t launch_strips(int precision, const StripPlan& p, double eps2, const IParticles& ip,
+                          const JStream& js, const Epilogue& ep, double* scratch, int sms, int mode,
+                          double* dst, long long ld, cudaStream_t stream);
+cudaError_t configure_strips();
 // Kernel attributes that must be set once per device, outside stream capture.
 cudaError_t configure_kernels();
 

@@ -1,0 +1,82 @@
+"""Newton-3 strips against the oracle at the edges of their units: batches of 32
+sources, row blocks of 32 x (receivers per lane), strips of one unit or none,
+and the sizes where the default takes them."""
+import os
+
+import numpy as np
+import pytest
+
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+FP64, FP32C = 0, 1
+SIZES = [1, 2, 31, 32, 33, 127, 129, 191, 193, 255, 257, 319, 321, 511, 513, 1000, 2049, 4096]
+
+
+def check(a, ref, prec):
+    """The bounds of the other force tests: FP64 differs by summation order
+    (1e-12); FP32C by its pair arithmetic (median 1e-6, worst 1e-4)."""
+    e = rel_err(a, ref)
+    if prec == FP64:
+        assert e.max() <= 1e-12, e.max()
+    else:
+        assert np.median(e) <= 1e-6 and e.max() <= 1e-4, (np.median(e), e.max())
+
+
+@pytest.mark.parametrize("prec", [FP64, FP32C])
+@pytest.mark.parametrize("eps2", [0.0, 1e-4])
+def test_forced_strips_at_unit_edges(ctx, nbr, oracle, prec, eps2):
+    ctx.set_force_config(prec, 3, 8)
+    try:
+        for n in SIZES:
+            s = nbr.plummer(n, 40 + n)
+            ctx.upload(s)
+            a = ctx.forces(prec, eps2=eps2)
+            ref = oracle.accel(s["x"], s["y"], s["z"], s["m"], eps2=eps2, extended=True)
+            if n == 1:
+                assert not a.any()
+            else:
+                check(a, ref, prec)
+            np.testing.assert_array_equal(a, ctx.forces(prec, eps2=eps2))
+    finally:
+        ctx.set_force_config(prec)
+
+
+@pytest.mark.parametrize("prec", [FP64, FP32C])
+@pytest.mark.parametrize("n", [4097, 4100, 5119, 5121, 7681, 9984, 20481])
+def test_default_strips(ctx, nbr, oracle, prec, n):
+    s = nbr.plummer(n, n)
+    ctx.upload(s)
+    assert ctx.get_force_config(prec, 1e-6)[0] == 3
+    idx = np.unique(np.concatenate([np.arange(0, n, 37), [n - 1]]))
+    ref = oracle.accel_subset(s["x"], s["y"], s["z"], s["m"], idx, eps2=1e-6)
+    check(ctx.forces(prec, eps2=1e-6)[:, idx], ref, prec)
+    # the partial sums of several launches, accumulated: the same to rounding
+    os.environ["NBR_TEST_N3_SLICES"] = "3"
+    try:
+        check(ctx.forces(prec, eps2=1e-6)[:, idx], ref, prec)
+    finally:
+        del os.environ["NBR_TEST_N3_SLICES"]
+
+
+@pytest.mark.parametrize("prec,tol", [(FP64, 1e-11), (FP32C, 1e-6)])
+@pytest.mark.parametrize("scheme", ["kdk", "euler"])
+def test_strip_runs_between_other_kernels(ctx, nbr, oracle, prec, tol, scheme):
+    """A run in strips leaves no FP32C records: a large-kernel evaluation after
+    it, and a run after that, see the moved particles."""
+    n, eps2 = 4500, 1e-4
+    s = nbr.plummer(n, 3)
+    ctx.upload(s)
+    ctx.run(prec, nbr.KDK if scheme == "kdk" else nbr.EULER, 2, 1e-3, 3, eps2=eps2)
+    advance = oracle.kdk if scheme == "kdk" else oracle.euler
+    want = advance(s, 1e-3, 3, eps2=eps2)
+    got = ctx.download()
+    for k in ("x", "y", "z", "vx", "vy", "vz"):
+        assert np.abs(got[k] - want[k]).max() <= tol, k
+    ctx.set_force_config(prec, 4, 4)
+    try:
+        a = ctx.forces(prec, eps2=eps2)
+    finally:
+        ctx.set_force_config(prec)
+    check(a, oracle.accel(got["x"], got["y"], got["z"], s["m"], eps2=eps2, extended=True), prec)
