@@ -638,11 +638,33 @@ int kick_drift_system(nbr_ctx* c, bool pack, double kick, double drift, bool use
 }
 
 // Softened potential of the uploaded system on the context stream: phi into
-// dphi (device, may be null) and U = 1/2 sum m_i phi_i into *dU (device).
-// Uses red[red_off ..] for the per-chunk sums.
+// dphi (device, may be null) and U = 1/2 sum m_i phi_i as *dU (device) times
+// *factor.  Without phi the pairs are evaluated once each (launch_energy).
+// Uses red[red_off ..] for the per-chunk sums: at most potential_sums(c) + 16.
+size_t potential_sums(const nbr_ctx* c) {
+  return std::max<size_t>((c->sys.n + 127) / 128, (size_t)kEnergyStrips * c->sms);
+}
 int potential_system(nbr_ctx* c, double G, double eps2, double* dphi, size_t red_off,
-                     double** dU) {
+                     double** dU, double* factor) {
   SysState& s = c->sys;
+  const int a = s.cur;
+  IParticles ip{s.pos[a][0], s.pos[a][1], s.pos[a][2], s.mass, (long long)s.n};
+  JStream js{s.pos[a][0], s.pos[a][1], s.pos[a][2], s.mass, nullptr, nullptr, s.ntiles, 0, -1};
+  pipeline_params(js);
+  NBR_CHECKED_ONLY(ip.len = (long long)(s.cap + kRangeSlack); js.len = (long long)s.cap;)
+  if (!dphi && (long long)s.n <= kEnergyMaxN) {
+    cudaError_t e = c->scr.need_red(red_off + potential_sums(c) + 16);
+    if (e != cudaSuccess) return cuda_fail(c, e, "potential scratch");
+    double* sums = c->scr.red + red_off;
+    int strips = 0;
+    e = launch_energy((long long)s.n, eps2, ip, js, c->d_err, sums, c->sms, &strips, c->stream);
+    if (e == cudaSuccess) e = launch_rowsum(sums, strips, 1, sums + strips, c->stream);
+    if (e != cudaSuccess) return cuda_fail(c, e, "energy launch");
+    *dU = sums + strips;
+    *factor = -G * kInvDistScale;
+    return NBR_OK;
+  }
+  *factor = 1.0;
   const ForceConfig pc{kPotNI, kPotWarps, 0};
   int split = auto_split(kFP64, eps2, pc, (long long)s.n, s.ntiles, c->sms);
   split = std::max(1, std::min(split, s.ntiles));
@@ -653,10 +675,6 @@ int potential_system(nbr_ctx* c, double G, double eps2, double* dphi, size_t red
   const int chunks = (int)(((long long)s.n + chunk - 1) / chunk);
   cudaError_t e = c->scr.need_red(red_off + (size_t)chunks + 16);
   if (e != cudaSuccess) return cuda_fail(c, e, "potential scratch");
-  const int a = s.cur;
-  IParticles ip{s.pos[a][0], s.pos[a][1], s.pos[a][2], s.mass, (long long)s.n};
-  JStream js{s.pos[a][0], s.pos[a][1], s.pos[a][2], s.mass, nullptr, nullptr, s.ntiles, 0, -1};
-  pipeline_params(js);
   PotentialOut po{};
   po.G = G;
   po.phi = dphi;
@@ -666,7 +684,6 @@ int potential_system(nbr_ctx* c, double G, double eps2, double* dphi, size_t red
   po.n_pad = (long long)s.n_pad;
   po.err = c->d_err;
   NBR_CHECKED_ONLY(
-      ip.len = (long long)(s.cap + kRangeSlack); js.len = (long long)s.cap;
       po.part_len = (long long)c->scr.part_cap; po.cnt_len = (long long)c->scr.cnt_cap;
       po.blocksum_len = (long long)(c->scr.red_cap - red_off);)
   e = launch_potential(split, ip, js, po, eps2, c->stream);
@@ -681,9 +698,9 @@ int diag_system(nbr_ctx* c, double G, double eps2, nbr_diag* out) {
   SysState& s = c->sys;
   const int a = s.cur;
   const int nb = (int)((s.n + 127) / 128);
-  // moments (8 x nb), their sums (16), then the potential's chunk sums (<= nb)
-  // and U: sized once here so that nothing below reallocates.
-  cudaError_t e = c->scr.need_red((size_t)nb * 10 + 48);
+  // moments (8 x nb), their sums (16), then the potential's sums and U: sized
+  // once here so that nothing below reallocates.
+  cudaError_t e = c->scr.need_red((size_t)nb * 9 + 32 + potential_sums(c));
   if (e != cudaSuccess) return cuda_fail(c, e, "diag scratch");
   double* part = c->scr.red;
   double* res = c->scr.red + (size_t)nb * 8;
@@ -691,8 +708,8 @@ int diag_system(nbr_ctx* c, double G, double eps2, nbr_diag* out) {
                      s.vel[0], s.vel[1], s.vel[2], s.mass, part, c->stream);
   if (e == cudaSuccess) e = launch_rowsum(part, nb, 8, res, c->stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "diagnostics");
-  double* dU = nullptr;
-  int rc = potential_system(c, G, eps2, nullptr, (size_t)nb * 9 + 16, &dU);
+  double *dU = nullptr, factor = 1.0;
+  int rc = potential_system(c, G, eps2, nullptr, (size_t)nb * 9 + 16, &dU, &factor);
   if (rc) return rc;
   double h[9];
   e = cudaMemcpyAsync(h, res, 8 * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
@@ -706,7 +723,7 @@ int diag_system(nbr_ctx* c, double G, double eps2, nbr_diag* out) {
   out->P[0] = h[1]; out->P[1] = h[2]; out->P[2] = h[3];
   out->L[0] = h[4]; out->L[1] = h[5]; out->L[2] = h[6];
   out->M = h[7];
-  out->U = h[8];
+  out->U = factor * h[8];
   out->E = out->T + out->U;
   return NBR_OK;
 }
@@ -1194,8 +1211,8 @@ int nbr_potential(nbr_ctx* c, double G, double eps2, double* phi, double* U) {
   // phi goes to the (otherwise idle) acceleration x array only when requested.
   double* dphi = phi ? s.acc[0] : nullptr;
   if (phi) c->acc_ok = false;
-  double* dU = nullptr;
-  int rc = potential_system(c, G, eps2, dphi, 0, &dU);
+  double *dU = nullptr, factor = 1.0;
+  int rc = potential_system(c, G, eps2, dphi, 0, &dU, &factor);
   if (rc) return rc;
   double u = 0.0;
   cudaError_t e = cudaMemcpyAsync(&u, dU, sizeof(double), cudaMemcpyDeviceToHost, c->stream);
@@ -1205,7 +1222,7 @@ int nbr_potential(nbr_ctx* c, double G, double eps2, double* phi, double* U) {
   if (e != cudaSuccess) return cuda_fail(c, e, "potential");
   rc = check_device_error(c);
   if (rc) return rc;
-  if (U) *U = u;
+  if (U) *U = factor * u;
   return NBR_OK;
 }
 

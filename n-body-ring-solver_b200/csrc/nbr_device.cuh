@@ -119,6 +119,28 @@ __device__ __forceinline__ double inv_cube(double r2) {
   return (y2 * y) * c;
 }
 
+// r^-1 / kInvDistScale for r2 = r^2, by the series of inv_cube:
+//     r^-1 = y (1 - h)^(-1/2) = y (1 + 1/2 h + 3/8 h^2 + ...)
+//          = 3/8 y (u^2 + 20/9),   u = h + 2/3 = 5/3 - r2 y^2,
+// the next term below 5/16 (1.9e-6)^3 = 2.1e-18; 20/9 and 3/8 are rounded to
+// the doubles whose product is nearest 1 at h = 0 (2e-17).  Four FP64
+// operations and one MUFU.  Only for normal r2: a caller whose sums stay
+// finite where r2 is subnormal takes rsqrt() there (see tiny_r2).
+constexpr double kInvDistScale = 0.37499999999999994;
+__device__ __forceinline__ double inv_dist(double r2) {
+  const double y = rsqrt_seed64(r2);
+  const double u = fma(-clamp_finite64(r2), y * y, 1.6666666666666665);
+  return y * fma(u, u, 2.2222222222222228);
+}
+// High word of r2 >= 0: below kTinyHi if r2 is zero or subnormal.
+constexpr int kTinyHi = 0x00100000;
+// inv_dist for any r2; EXCL: 0 for r2 = 0.
+template <bool EXCL>
+__device__ __noinline__ double inv_dist_tiny(double r2) {
+  if (EXCL && !(r2 > 0.0)) return 0.0;
+  return rsqrt(r2) * (1.0 / kInvDistScale);
+}
+
 // Knuth TwoSum of the packed pair (hi + p): hi <- rounded sum, lo += the
 // rounding error.  Six packed adds; exact error term for round-to-nearest.
 __device__ __forceinline__ void two_sum2(u64& hi, u64& lo, u64 p) {

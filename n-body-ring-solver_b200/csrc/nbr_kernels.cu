@@ -44,6 +44,7 @@
 #include <mutex>
 #include <queue>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 namespace nbr {
@@ -1465,8 +1466,8 @@ __device__ __forceinline__ void block_reduce_store(double (&v)[W], double* out) 
 // Softened potential phi_i = -G sum_{j != i} m_j / sqrt(r^2 + eps2), FP64, with
 // the structure of the FP64 force kernel (receivers in registers, source tiles
 // through the bulk-copy ring, j range split over gridDim.y with a
-// deterministic last-CTA reduction).  Per pair: 3 sub, 3 fma, CUDA's
-// rsqrt(double), 1 fma; the self pair is skipped by index (with eps2 > 0 it
+// deterministic last-CTA reduction).  Per pair: 3 sub, 3 fma, 4 operations of
+// inv_dist, 1 fma; the self pair is skipped by index (with eps2 > 0 it
 // would add m_i / eps).  The last CTA of each receiver chunk writes phi and
 // the chunk's sum of 1/2 m_i phi_i (fixed-order tree: deterministic).
 template <int NI, int WARPS, bool EXCL>
@@ -1512,8 +1513,14 @@ __global__ void __launch_bounds__(WARPS * 32)
     const double* sm = sz + kTile;
     const int jself = i0 - tcur * kTile;  // receiver k's own index in this tile is jself + 32 k
     ++tcur;
-#pragma unroll 2
-    for (int j = 0; j < kTile; ++j) {
+    // Every pair by inv_dist, then, where a r2 was zero or subnormal, the whole
+    // tile again with the limit's own arithmetic.
+    const bool own = jself - lane > -32 * NI && jself - lane < kTile;
+    double keep[NI];
+#pragma unroll
+    for (int k = 0; k < NI; ++k) keep[k] = ph[k];
+    int lo = 0x7fffffff;
+    auto pairs = [&](auto self_pair, auto limit, int j) {
       const double xj = sx[j], yj = sy[j], zj = sz[j], mj = sm[j];
 #pragma unroll
       for (int k = 0; k < NI; ++k) {
@@ -1521,11 +1528,28 @@ __global__ void __launch_bounds__(WARPS * 32)
         double r2 = fma(dx, dx, eps2);
         r2 = fma(dy, dy, r2);
         r2 = fma(dz, dz, r2);
-        double y = rsqrt(r2);
-        if (EXCL) y = r2 > 0.0 ? y : 0.0;
-        y = (j == jself + 32 * k) ? 0.0 : y;
+        const bool self = decltype(self_pair)::value && j == jself + 32 * k;
+        const int hi = __double2hiint(r2);
+        if (!decltype(limit)::value) lo = min(lo, self ? 0x7fffffff : hi);
+        double y = decltype(limit)::value && hi < kTinyHi ? inv_dist_tiny<EXCL>(r2) : inv_dist(r2);
+        if (self) y = 0.0;
         ph[k] = fma(mj, y, ph[k]);
       }
+    };
+    const std::true_type yes;
+    const std::false_type no;
+    if (own) {
+#pragma unroll 2
+      for (int j = 0; j < kTile; ++j) pairs(yes, no, j);
+    } else {
+#pragma unroll 4
+      for (int j = 0; j < kTile; ++j) pairs(no, no, j);
+    }
+    if (lo < kTinyHi) {
+#pragma unroll
+      for (int k = 0; k < NI; ++k) ph[k] = keep[k];
+#pragma unroll 1
+      for (int j = 0; j < kTile; ++j) pairs(yes, yes, j);
     }
   };
   if (!tile_pipeline(bars, t1 - t0, js, po.err, issue, body)) return;
@@ -1561,7 +1585,7 @@ __global__ void __launch_bounds__(WARPS * 32)
   for (int k = 0; k < NI; ++k) {
     const long long i = ibase + 32 * k;
     if (i < ip.n) {
-      const double p = -po.G * ph[k];
+      const double p = -po.G * (kInvDistScale * ph[k]);
       if (po.phi) po.phi[i] = p;
       half += 0.5 * ip.m[i] * p;
     }

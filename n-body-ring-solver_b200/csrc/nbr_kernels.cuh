@@ -263,6 +263,14 @@ cudaError_t launch_strips(int precision, const StripPlan& p, double eps2, const 
                           const JStream& js, const Epilogue& ep, double* scratch, int sms, int mode,
                           double* dst, long long ld, cudaStream_t stream);
 cudaError_t configure_strips();
+// Sums of m_i m_j / r over the unordered pairs of the particles, over
+// kInvDistScale, one per strip: at most kEnergyStrips x sms, the number used
+// into *count.  n up to kEnergyMaxN (32-bit unit numbers).
+constexpr int kEnergyStrips = 2 * kStripWarps;
+constexpr long long kEnergyWideN = 8192;
+constexpr long long kEnergyMaxN = 1LL << 21;
+cudaError_t launch_energy(long long n, double eps2, const IParticles& ip, const JStream& js, int* err,
+                          double* sums, int sms, int* count, cudaStream_t stream);
 // Kernel attributes that must be set once per device, outside stream capture.
 cudaError_t configure_kernels();
 

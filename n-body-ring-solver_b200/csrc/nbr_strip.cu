@@ -363,6 +363,103 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
   }
 }
 
+// The potential energy of the system over -G kInvDistScale: the units of the
+// strips, each unordered pair once (in a block's own batches twice, at half the
+// mass), with no reaction to carry: a step's source is read from the warp's
+// staging buffer by all lanes.  Per pair 3 differences, 3 fma, 4 operations of
+// inv_dist and 1 fma = 11, so 5.5 per ordered pair, against 11 in k_potential_f64,
+// which also gives every particle's potential.  One sum per strip, lanes in
+// xor order.  us per diagnostics call on B200, every ordered pair with
+// rsqrt(double) / this: N = 2000 125 / 65, 16000 377 / 167, 65500 4198 / 1657, 262144
+// 64535 / 24979 (81 % of the FP64 pipe).  8 receivers per lane in one CTA of 8
+// warps per SM (two such CTAs spill: 27495); below kEnergyWideN 4 in two CTAs,
+// for more units.
+template <int NI, bool EXCL>
+__global__ void __launch_bounds__(kStripWarps * 32, NI == 4 ? 2 : 1)
+    k_strip_energy(const IParticles ip, const JStream js, const StripPlan sp, const double eps2,
+                   double* sums, int* err) {
+  constexpr int TB = NI;
+  __shared__ double2 src[kStripWarps][32][2];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = warp * gridDim.x + blockIdx.x;
+  if (g >= sp.strips) return;
+  int u = strip_start(sp, g);
+  const int u_end = strip_start(sp, g + 1);
+  double total = 0.0;
+  for (int r = strip_row(sp, u); u < u_end; ++r) {
+    const int b0 = r * TB + (u - strip_prefix(sp, r));
+    const int b1 = min(sp.batches, b0 + (u_end - u));
+    u += b1 - b0;
+    const long long ibase = (long long)r * (32 * NI) + lane;
+    if (!NBR_IN((long long)(r + 1) * (32 * NI) - 1, ip.len, err) ||
+        !NBR_IN(32LL * b1 - 1, js.len, err))
+      return;
+    double xi[NI], yi[NI], zi[NI], ph[NI];
+#pragma unroll
+    for (int k = 0; k < NI; ++k) {
+      const long long i = ibase + 32 * k;
+      xi[k] = ip.x[i]; yi[k] = ip.y[i]; zi[k] = ip.z[i];
+      ph[k] = 0.0;
+    }
+    long long j = 32LL * b0 + lane;
+    double qx = js.x[j], qy = js.y[j], qz = js.z[j], qm = js.m[j];
+#pragma unroll 1
+    for (int b = b0; b < b1; ++b) {
+      const bool own = b < (r + 1) * TB;
+      __syncwarp();
+      src[warp][lane][0] = make_double2(qx, qy);
+      src[warp][lane][1] = make_double2(qz, own ? 0.5 * qm : qm);
+      __syncwarp();
+      j += 32;
+      if (b + 1 < b1) { qx = js.x[j]; qy = js.y[j]; qz = js.z[j]; qm = js.m[j]; }
+      // Every pair by inv_dist, then, where a r2 was zero or subnormal, the
+      // whole batch again with the limit's own arithmetic.  In the block's own
+      // batches receiver kself of lane `step` is the source itself: no pair.
+      const int kself = own ? b - r * TB : -1;
+      double keep[NI];
+#pragma unroll
+      for (int k = 0; k < NI; ++k) keep[k] = ph[k];
+      int lo = 0x7fffffff;
+      auto pairs = [&](auto self_pair, auto limit, int step) {
+        const double2 a = src[warp][step][0], c = src[warp][step][1];
+#pragma unroll
+        for (int k = 0; k < NI; ++k) {
+          const double dx = a.x - xi[k], dy = a.y - yi[k], dz = c.x - zi[k];
+          double r2 = fma(dx, dx, eps2);
+          r2 = fma(dy, dy, r2);
+          r2 = fma(dz, dz, r2);
+          const bool self = decltype(self_pair)::value && k == kself && step == lane;
+          const int hi = __double2hiint(r2);
+          if (!decltype(limit)::value) lo = min(lo, self ? 0x7fffffff : hi);
+          double v = decltype(limit)::value && hi < kTinyHi ? inv_dist_tiny<EXCL>(r2) : inv_dist(r2);
+          if (self) v = 0.0;
+          ph[k] = fma(c.y, v, ph[k]);
+        }
+      };
+      const std::true_type yes;
+      const std::false_type no;
+      if (own) {
+#pragma unroll 2
+        for (int step = 0; step < 32; ++step) pairs(yes, no, step);
+      } else {
+#pragma unroll 4
+        for (int step = 0; step < 32; ++step) pairs(no, no, step);
+      }
+      if (lo < kTinyHi) {
+#pragma unroll
+        for (int k = 0; k < NI; ++k) ph[k] = keep[k];
+#pragma unroll 1
+        for (int step = 0; step < 32; ++step) pairs(yes, yes, step);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < NI; ++k) total = fma(ip.m[ibase + 32 * k], ph[k], total);
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) total += __shfl_xor_sync(0xffffffffu, total, off);
+  if (lane == 0) sums[g] = total;
+}
+
 // Adds the partial sums of a batch's 32 particles, one per lane: its row block's
 // strips, then the reactions from the row blocks before it, spread over the
 // CTA's warps (a particle's chain of loads is what takes the time on a small
@@ -542,6 +639,21 @@ const void* strip_fn(int precision, int ni, bool excl, bool fine) {
 size_t strip_smem(int ni) { return (size_t)kStripWarps * 96 * ni * sizeof(double); }
 
 }  // namespace
+
+cudaError_t launch_energy(long long n, double eps2, const IParticles& ip, const JStream& js, int* err,
+                          double* sums, int sms, int* count, cudaStream_t st) {
+  const int ni = n < kEnergyWideN ? 4 : 8, grid = (ni == 4 ? 2 : 1) * sms;
+  const StripPlan p = strip_plan(kFP64, n, 0, 1 << 30, grid, ni);
+  *count = p.strips;
+  if (eps2 == 0.0) {
+    if (ni == 4) k_strip_energy<4, true><<<grid, kStripWarps * 32, 0, st>>>(ip, js, p, 0.0, sums, err);
+    else k_strip_energy<8, true><<<grid, kStripWarps * 32, 0, st>>>(ip, js, p, 0.0, sums, err);
+  } else {
+    if (ni == 4) k_strip_energy<4, false><<<grid, kStripWarps * 32, 0, st>>>(ip, js, p, eps2, sums, err);
+    else k_strip_energy<8, false><<<grid, kStripWarps * 32, 0, st>>>(ip, js, p, eps2, sums, err);
+  }
+  return cudaGetLastError();
+}
 
 cudaError_t configure_strips() {
   cudaError_t e = cudaSuccess;

@@ -80,3 +80,36 @@ def test_strip_runs_between_other_kernels(ctx, nbr, oracle, prec, tol, scheme):
     finally:
         ctx.set_force_config(prec)
     check(a, oracle.accel(got["x"], got["y"], got["z"], s["m"], eps2=eps2, extended=True), prec)
+
+
+@pytest.mark.parametrize("eps2", [0.0, 1e-4])
+def test_energy_by_pairs_equals_the_potential(ctx, nbr, oracle, eps2):
+    """diagnostics() evaluates each pair once, potential() every ordered pair:
+    the same sum to rounding, and the oracle's, at the edges of the units."""
+    for n in [1, 2, 31, 33, 127, 129, 255, 257, 1000, 4097, 8191, 8193, 12345]:
+        s = nbr.plummer(n, n)
+        ctx.upload(s)
+        d = ctx.diagnostics(eps2=eps2)
+        U, phi = ctx.potential(eps2=eps2, per_particle=True)
+        assert abs(d["U"] - U) <= 1e-13 * abs(U), n
+        assert abs(0.5 * (s["m"] * phi).sum() - U) <= 1e-13 * abs(U), n
+        if n <= 4097:
+            ref = oracle.energy(s, eps2=eps2)["U"]
+            assert abs(d["U"] - ref) <= 1e-13 * abs(ref), n
+
+
+# r^2 subnormal (its own rounding is the reference's too), tiny, ordinary, and
+# overflowing (no contribution): 4 roundings of the inverse distance and the
+# two masses' products stay within 1e-15.
+@pytest.mark.parametrize("d", [1e-160, 3e-157, 1e-150, 1e-100, 1.0, 1e100, 1e160])
+def test_energy_of_an_extreme_pair(ctx, d):
+    z = np.zeros(2)
+    with np.errstate(over="ignore", under="ignore"):
+        r2 = np.float64(d) * np.float64(d)
+        want = -0.25 / np.sqrt(r2) if np.isfinite(r2) else 0.0
+    ctx.upload({"x": np.array([0.0, d]), "y": z, "z": z, "m": np.array([0.5, 0.5])})
+    for U in (ctx.diagnostics()["U"], ctx.potential(), ctx.potential(per_particle=True)[0]):
+        assert abs(U - want) <= 1e-15 * abs(want)
+    # a coincident pair is skipped without softening
+    ctx.upload({"x": z, "y": z, "z": z, "m": np.array([0.5, 0.5])})
+    assert ctx.diagnostics()["U"] == 0.0 and ctx.potential(per_particle=True)[0] == 0.0
