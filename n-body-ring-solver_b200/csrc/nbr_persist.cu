@@ -12,18 +12,27 @@
 //    shared memory with L2 loads, its W warps (8 or 16) split the sources W
 //    ways and the F lane groups of each warp split them again
 //    (k_force_small's layout), and the partial sums are combined in a fixed
-//    order (xor shuffles, then the warps in order): deterministic;
-//  * the CTA applies the fused kick/drift to its receivers, whose velocities
-//    (and, FP32C, positions) stay in shared memory for the run, writes their
-//    positions to the next buffer, and all CTAs meet at one grid barrier
-//    before the next evaluation reads it.
+//    order (lane_sums, then the warps in order): deterministic;
+//  * the CTA applies the fused kick/drift to its receivers, one thread per
+//    receiver and axis, whose velocities (and, FP32C, positions) stay in shared
+//    memory for the run, writes their positions to the next buffer, and all
+//    CTAs meet at one grid barrier before the next evaluation reads it.
 //
 // The barrier is a 64-bit arrival counter that only grows; its wait is bounded
 // by %globaltimer (the context's wait limit) and gives up, with an error code
 // for the host, if the limit passes or another CTA has already recorded an
 // error.  The cooperative launch guarantees that all CTAs are resident, so no
-// CTA waits on one that cannot run.  FP64 pair arithmetic is k_force_f64's
-// (inv_cube): results equal the other FP64 kernels' up to summation order; the FP32C form (k_run_small_f32c) is described there.
+// CTA waits on one that cannot run.  (A flag per CTA, watched by a thread each,
+// instead of the counter took 2.5 us longer per step: 148 x 148 polls.)  FP64
+// pair arithmetic is k_force_f64's (inv_cube): results equal the other FP64
+// kernels' up to summation order; the FP32C form (k_run_small_f32c) is
+// described there.
+//
+// What bounds a step at N = 2048 is the latency between its phases as much as
+// the pairs (FP64: 3.9 us of pipe time in 7.8).  us per step on B200, with one
+// shuffle per value and lane bit, a thread per receiver and 4 receivers per
+// lane / now: FP64 N = 64 3.3 / 2.9, 1000 5.2 / 4.1, 2048 8.3 / 7.8, 3000 17.6 /
+// 14.4, 4096 22.3 / 20.4; FP32C N = 64 3.8 / 3.4, 1999 7.0 / 6.6, 4096 15.1 / 14.7.
 #include "nbr.h"
 #include "nbr_ctx.h"
 #include "nbr_device.cuh"
@@ -110,6 +119,39 @@ __device__ bool grid_barrier(unsigned long long* bar, int* err, unsigned long lo
   return s_ok != 0;
 }
 
+// Sums of v[0 .. V) over the lanes that differ in the bits 16, 8, .. G of the
+// lane number, spread over those lanes: at each bit a lane keeps one half of
+// its values and hands the other half to its partner, so V values cost about V
+// exchanges in all instead of V at every bit.  Calls put(index, sum) for the
+// values that end up on this lane.  Fixed order: deterministic.
+template <int V, int OFF, int G, class Put>
+__device__ __forceinline__ void lane_sums(const double* v, int lane, int base, int cnt, Put put) {
+  if constexpr (OFF < G) {
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+      if (i < cnt) put(base + i, v[i]);
+  } else {
+    constexpr int H = (V + 1) / 2;
+    const bool up = (lane & OFF) != 0;
+    double w[H];
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+      const double lo = v[i], hi = i + H < V ? v[i + H] : 0.0;
+      w[i] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, OFF);
+    }
+    lane_sums<H, OFF / 2, G>(w, lane, up ? base + H : base, up ? cnt - H : min(cnt, H), put);
+  }
+}
+
+// Sources in shared memory, padded to a whole number for each of the S ways
+// they are split, so that every lane runs the same trips (a ragged end cost a
+// step of N = 1999 8 %).  The padding is massless and far away, and written
+// once per run: FP64 so far that r^2 overflows and the pair contributes 0
+// (inv_cube), FP32C where r^2 and r^-3 stay finite.
+__host__ __device__ inline int padded_sources(int n, int S) { return (n + S - 1) / S * S; }
+constexpr double kPadFar64 = 1e200;
+constexpr float kPadFar32 = 1e15f;
+
 // W warps per CTA (8 or 16), F lane groups per warp, kPNI receivers per lane.
 template <int F, int W, int kPNI, bool EXCL>
 __global__ void __launch_bounds__(W * 32, 1) k_run_small_f64(const PersistArgs A) {
@@ -120,7 +162,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_run_small_f64(const PersistArgs A
   constexpr int S = kPWarps * F;   // ways the sources are split
   extern __shared__ __align__(16) double smem_d[];
   const int n = A.n;
-  const int ns = (n + 1) & ~1;
+  const int ns = padded_sources(n, S);
   double* sx = smem_d;
   double* sy = sx + ns;
   double* sz = sy + ns;
@@ -131,7 +173,10 @@ __global__ void __launch_bounds__(W * 32, 1) k_run_small_f64(const PersistArgs A
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gl = lane % G, grp = lane / G;
 
-  for (int j = threadIdx.x; j < n; j += kPThreads) sm[j] = A.m[j];
+  for (int j = threadIdx.x; j < ns; j += kPThreads) {
+    sm[j] = j < n ? A.m[j] : 0.0;
+    if (j >= n) sx[j] = sy[j] = sz[j] = kPadFar64;
+  }
   int cur = A.cur0;
   unsigned long long nbar = 0;  // grid barriers passed
 
@@ -170,8 +215,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_run_small_f64(const PersistArgs A
     const double* X = A.px[cur];
     const double* Y = A.py[cur];
     const double* Z = A.pz[cur];
-    // 16-byte L2 loads, several in flight per thread before the stores (the
-    // arrays hold at least ns entries: n_pad is a multiple of 1024)
+    // 16-byte L2 loads, several in flight per thread before the stores
     {
       const double2* X2 = reinterpret_cast<const double2*>(X);
       const double2* Y2 = reinterpret_cast<const double2*>(Y);
@@ -180,11 +224,13 @@ __global__ void __launch_bounds__(W * 32, 1) k_run_small_f64(const PersistArgs A
       double2* sy2 = reinterpret_cast<double2*>(sy);
       double2* sz2 = reinterpret_cast<double2*>(sz);
 #pragma unroll 4
-      for (int j = threadIdx.x; j < ns / 2; j += kPThreads) {
+      for (int j = threadIdx.x; j < (n + 1) / 2; j += kPThreads) {
         const double2 a = __ldcg(X2 + j), b = __ldcg(Y2 + j), c = __ldcg(Z2 + j);
-        sx2[j] = a;
-        sy2[j] = b;
-        sz2[j] = c;
+        if (2 * j + 1 < n) {
+          sx2[j] = a; sy2[j] = b; sz2[j] = c;
+        } else {
+          sx[2 * j] = a.x; sy[2 * j] = b.x; sz[2 * j] = c.x;
+        }
       }
     }
     __syncthreads();
@@ -202,7 +248,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_run_small_f64(const PersistArgs A
         ax[k] = ay[k] = az[k] = 0.0;
       }
 #pragma unroll 4
-      for (int j = warp * F + grp; j < n; j += S) {
+      for (int j = warp * F + grp; j < ns; j += S) {
         const double xj = sx[j], yj = sy[j], zj = sz[j], mj = sm[j];
 #pragma unroll
         for (int k = 0; k < kPNI; ++k) {
@@ -217,48 +263,33 @@ __global__ void __launch_bounds__(W * 32, 1) k_run_small_f64(const PersistArgs A
         }
       }
       // lane groups of the warp, then the warps in order
+      double v[3 * kPNI];
 #pragma unroll
-      for (int off = G; off < 32; off <<= 1) {
-#pragma unroll
-        for (int k = 0; k < kPNI; ++k) {
-          ax[k] += __shfl_xor_sync(0xffffffffu, ax[k], off);
-          ay[k] += __shfl_xor_sync(0xffffffffu, ay[k], off);
-          az[k] += __shfl_xor_sync(0xffffffffu, az[k], off);
-        }
-      }
-      if (grp == 0) {
-#pragma unroll
-        for (int k = 0; k < kPNI; ++k) {
-          double* r = red + ((size_t)warp * RPC + gl + G * k) * 3;
-          r[0] = ax[k]; r[1] = ay[k]; r[2] = az[k];
-        }
-      }
+      for (int k = 0; k < kPNI; ++k) { v[3 * k] = ax[k]; v[3 * k + 1] = ay[k]; v[3 * k + 2] = az[k]; }
+      lane_sums<3 * kPNI, 16, G>(v, lane, 0, 3 * kPNI, [&](int i, double sum) {
+        const int k = i / 3;
+        red[((size_t)warp * RPC + gl + G * k) * 3 + (i - 3 * k)] = sum;
+      });
       __syncthreads();
-      if (threadIdx.x < RPC) {
-        const int t = threadIdx.x, i = base + t;
-        double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+      // one thread per receiver and axis: the epilogue of the large kernels,
+      // a -> acc, v += kick a, x' = x + drift v (Euler: drift with the old velocity)
+      if (threadIdx.x < 3 * RPC) {
+        const int t = threadIdx.x / 3, d = threadIdx.x - 3 * t, i = base + t;
+        double a = 0.0;
 #pragma unroll
-        for (int w = 0; w < kPWarps; ++w) {
-          const double* r = red + ((size_t)w * RPC + t) * 3;
-          a0 += r[0]; a1 += r[1]; a2 += r[2];
-        }
-        a0 *= kInvCubeScale; a1 *= kInvCubeScale; a2 *= kInvCubeScale;
+        for (int w = 0; w < kPWarps; ++w) a += red[(size_t)w * RPC * 3 + threadIdx.x];
         if (t < A.cs && i < n) {
-          // the epilogue of the large kernels: a -> acc, v += kick a, x' = x + drift v
-          // (Euler: drift with the old velocity)
-          const double gx = A.G * a0, gy = A.G * a1, gz = A.G * a2;
-          A.ax[i] = gx; A.ay[i] = gy; A.az[i] = gz;
-          double* v = svel + ((size_t)round * RPC + t) * 3;
-          const double ux = v[0], uy = v[1], uz = v[2];
-          const double vx = ux + kd.x * gx, vy = uy + kd.x * gy, vz = uz + kd.x * gz;
-          v[0] = vx; v[1] = vy; v[2] = vz;
-          const bool euler = A.mode == 2;
-          A.px[1 - cur][i] = sx[i] + kd.y * (euler ? ux : vx);
-          A.py[1 - cur][i] = sy[i] + kd.y * (euler ? uy : vy);
-          A.pz[1 - cur][i] = sz[i] + kd.y * (euler ? uz : vz);
+          const double gx = A.G * (kInvCubeScale * a);
+          if (e + 1 == A.evals) (d == 0 ? A.ax : d == 1 ? A.ay : A.az)[i] = gx;
+          double* vel = svel + ((size_t)round * RPC + t) * 3 + d;
+          const double ux = *vel, vx = ux + kd.x * gx;
+          *vel = vx;
+          const double* x = d == 0 ? sx : d == 1 ? sy : sz;
+          double* xn = d == 0 ? A.px[1 - cur] : d == 1 ? A.py[1 - cur] : A.pz[1 - cur];
+          xn[i] = x[i] + kd.y * (A.mode == 2 ? ux : vx);
         }
       }
-      __syncthreads();  // red is reused by the next chunk
+      if (c + gridDim.x < A.chunks) __syncthreads();  // red is reused by the next chunk
     }
     if (e + 1 < A.evals) {
       if (e == A.skip_barrier && blockIdx.x == 0) return;  // test hook: never arrives
@@ -266,6 +297,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_run_small_f64(const PersistArgs A
     }
     cur ^= 1;
   }
+  __syncthreads();  // the last evaluation's velocities
   for (int c = blockIdx.x, r = 0; c < A.chunks; c += gridDim.x, ++r)
     for (int t = threadIdx.x; t < A.cs; t += kPThreads) {
       const int i = c * A.cs + t;
@@ -295,7 +327,7 @@ __global__ void __launch_bounds__(kPW32 * 32, 1) k_run_small_f32c(const PersistA
   extern __shared__ __align__(16) unsigned char smem_b[];
   __shared__ double s_org[W][3];
   __shared__ double s_o[3];
-  const int n = A.n, ns = (n + 1) & ~1;
+  const int n = A.n, n2 = (n + 1) / 2, ns = padded_sources(n, S);
   ulonglong2* rxy = reinterpret_cast<ulonglong2*>(smem_b);  // [ns] (x, x, y, y)
   ulonglong2* rzm = rxy + ns;                               // [ns] (z, z, -1.5 m, -1.5 m)
   u64* rb = reinterpret_cast<u64*>(rzm + ns);               // [ns] (2.5 m, 2.5 m)
@@ -307,11 +339,13 @@ __global__ void __launch_bounds__(kPW32 * 32, 1) k_run_small_f32c(const PersistA
   const int gl = lane % G, grp = lane / G;
   const float e2f = (float)A.eps2;
   const u64 EPS2 = pack2(e2f, e2f);
+  const double inv_n = 1.0 / n;
 
   for (int j = threadIdx.x; j < ns; j += NT) {
     const double m = j < n ? A.m[j] : 0.0;
     const float fa = __double2float_rn(-1.5 * m), fb = __double2float_rn(2.5 * m);
-    rzm[j] = make_ulonglong2(0ull, pack2(fa, fa));
+    rzm[j] = make_ulonglong2(pack2(kPadFar32, kPadFar32), pack2(fa, fa));
+    rxy[j] = make_ulonglong2(pack2(kPadFar32, kPadFar32), pack2(kPadFar32, kPadFar32));
     rb[j] = pack2(fb, fb);
   }
   int cur = A.cur0;
@@ -359,7 +393,7 @@ __global__ void __launch_bounds__(kPW32 * 32, 1) k_run_small_f32c(const PersistA
     for (int k = 0; k < kPLoads32; ++k) {
       const int j2 = threadIdx.x + k * NT;
       qx[k] = qy[k] = qz[k] = make_double2(0.0, 0.0);
-      if (j2 < ns / 2) {
+      if (j2 < n2) {
         qx[k] = __ldcg(X2 + j2); qy[k] = __ldcg(Y2 + j2); qz[k] = __ldcg(Z2 + j2);
         ox += qx[k].x; oy += qy[k].x; oz += qz[k].x;
         if (2 * j2 + 1 < n) { ox += qx[k].y; oy += qy[k].y; oz += qz[k].y; }
@@ -373,24 +407,27 @@ __global__ void __launch_bounds__(kPW32 * 32, 1) k_run_small_f32c(const PersistA
     }
     if (lane == 0) { s_org[warp][0] = ox; s_org[warp][1] = oy; s_org[warp][2] = oz; }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double a = 0.0, b = 0.0, cc = 0.0;
-      for (int w = 0; w < W; ++w) { a += s_org[w][0]; b += s_org[w][1]; cc += s_org[w][2]; }
-      s_o[0] = a / n; s_o[1] = b / n; s_o[2] = cc / n;
+    if (threadIdx.x < 3) {
+      double a = 0.0;
+#pragma unroll
+      for (int w = 0; w < W; ++w) a += s_org[w][threadIdx.x];
+      s_o[threadIdx.x] = a * inv_n;
     }
     __syncthreads();
     const double o0 = s_o[0], o1 = s_o[1], o2 = s_o[2];
 #pragma unroll
     for (int k = 0; k < kPLoads32; ++k) {
       const int j2 = threadIdx.x + k * NT;
-      if (j2 < ns / 2) {
+      if (j2 < n2) {
         const float x0 = __double2float_rn(qx[k].x - o0), x1 = __double2float_rn(qx[k].y - o0);
         const float y0 = __double2float_rn(qy[k].x - o1), y1 = __double2float_rn(qy[k].y - o1);
         const float z0 = __double2float_rn(qz[k].x - o2), z1 = __double2float_rn(qz[k].y - o2);
         rxy[2 * j2] = make_ulonglong2(pack2(x0, x0), pack2(y0, y0));
-        rxy[2 * j2 + 1] = make_ulonglong2(pack2(x1, x1), pack2(y1, y1));
         reinterpret_cast<u64*>(rzm + 2 * j2)[0] = pack2(z0, z0);
-        reinterpret_cast<u64*>(rzm + 2 * j2 + 1)[0] = pack2(z1, z1);
+        if (2 * j2 + 1 < n) {
+          rxy[2 * j2 + 1] = make_ulonglong2(pack2(x1, x1), pack2(y1, y1));
+          reinterpret_cast<u64*>(rzm + 2 * j2 + 1)[0] = pack2(z1, z1);
+        }
       }
     }
     __syncthreads();
@@ -408,8 +445,8 @@ __global__ void __launch_bounds__(kPW32 * 32, 1) k_run_small_f32c(const PersistA
         ZI[p] = pack2(__double2float_rn(r0[2] - o2), __double2float_rn(r1[2] - o2));
         AX[p] = AY[p] = AZ[p] = 0ull;
       }
-#pragma unroll 2
-      for (int j = warp * F + grp; j < n; j += S) {
+#pragma unroll 4  // N = 4096: 15.5 us per step unrolled by 2, 14.7 by 4
+      for (int j = warp * F + grp; j < ns; j += S) {
         const ulonglong2 q0 = rxy[j];
         const ulonglong2 q1 = rzm[j];
         const u64 bj = rb[j];
@@ -439,53 +476,34 @@ __global__ void __launch_bounds__(kPW32 * 32, 1) k_run_small_f32c(const PersistA
           AZ[p] = fma2(sv, dz, AZ[p]);
         }
       }
-      double ax[NI], ay[NI], az[NI];
+      double v[3 * NI];
 #pragma unroll
       for (int p = 0; p < IPAIR; ++p) {
         float l, h;
-        unpack2(AX[p], l, h); ax[2 * p] = l; ax[2 * p + 1] = h;
-        unpack2(AY[p], l, h); ay[2 * p] = l; ay[2 * p + 1] = h;
-        unpack2(AZ[p], l, h); az[2 * p] = l; az[2 * p + 1] = h;
+        unpack2(AX[p], l, h); v[6 * p] = l; v[6 * p + 3] = h;
+        unpack2(AY[p], l, h); v[6 * p + 1] = l; v[6 * p + 4] = h;
+        unpack2(AZ[p], l, h); v[6 * p + 2] = l; v[6 * p + 5] = h;
       }
-#pragma unroll
-      for (int off = G; off < 32; off <<= 1) {
-#pragma unroll
-        for (int k = 0; k < NI; ++k) {
-          ax[k] += __shfl_xor_sync(0xffffffffu, ax[k], off);
-          ay[k] += __shfl_xor_sync(0xffffffffu, ay[k], off);
-          az[k] += __shfl_xor_sync(0xffffffffu, az[k], off);
-        }
-      }
-      if (grp == 0) {
-#pragma unroll
-        for (int k = 0; k < NI; ++k) {
-          double* r = red + ((size_t)warp * RPC + gl + G * k) * 3;
-          r[0] = ax[k]; r[1] = ay[k]; r[2] = az[k];
-        }
-      }
+      lane_sums<3 * NI, 16, G>(v, lane, 0, 3 * NI, [&](int i, double sum) {
+        const int k = i / 3;
+        red[((size_t)warp * RPC + gl + G * k) * 3 + (i - 3 * k)] = sum;
+      });
       __syncthreads();
-      if (threadIdx.x < RPC) {
-        const int t = threadIdx.x, i = base + t;
-        double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+      if (threadIdx.x < 3 * RPC) {  // one thread per receiver and axis
+        const int t = threadIdx.x / 3, d = threadIdx.x - 3 * t, i = base + t;
+        double a = 0.0;
 #pragma unroll
-        for (int w = 0; w < W; ++w) {
-          const double* r = red + ((size_t)w * RPC + t) * 3;
-          a0 += r[0]; a1 += r[1]; a2 += r[2];
-        }
+        for (int w = 0; w < W; ++w) a += red[(size_t)w * RPC * 3 + threadIdx.x];
         if (t < A.cs && i < n) {
-          const double gx = A.G * a0, gy = A.G * a1, gz = A.G * a2;
-          A.ax[i] = gx; A.ay[i] = gy; A.az[i] = gz;
-          double* v = svel + ((size_t)round * RPC + t) * 3;
-          double* x = sp + (size_t)t * 3;
-          const double ux = v[0], uy = v[1], uz = v[2];
-          const double vx = ux + kd.x * gx, vy = uy + kd.x * gy, vz = uz + kd.x * gz;
-          v[0] = vx; v[1] = vy; v[2] = vz;
-          const bool euler = A.mode == 2;
-          const double nx = x[0] + kd.y * (euler ? ux : vx);
-          const double ny = x[1] + kd.y * (euler ? uy : vy);
-          const double nz = x[2] + kd.y * (euler ? uz : vz);
-          x[0] = nx; x[1] = ny; x[2] = nz;
-          A.px[1 - cur][i] = nx; A.py[1 - cur][i] = ny; A.pz[1 - cur][i] = nz;
+          const double gx = A.G * a;
+          if (e + 1 == A.evals) (d == 0 ? A.ax : d == 1 ? A.ay : A.az)[i] = gx;
+          double* vel = svel + ((size_t)round * RPC + t) * 3 + d;
+          double* x = sp + (size_t)t * 3 + d;
+          const double ux = *vel, vx = ux + kd.x * gx;
+          *vel = vx;
+          const double nx = *x + kd.y * (A.mode == 2 ? ux : vx);
+          *x = nx;
+          (d == 0 ? A.px[1 - cur] : d == 1 ? A.py[1 - cur] : A.pz[1 - cur])[i] = nx;
         }
       }
       __syncthreads();  // red and the receivers' positions are read again
@@ -515,7 +533,7 @@ const void* persist_fn32(int F, bool excl) {
 }
 
 size_t persist_smem32(int n, int F, int rounds) {
-  const int ns = (n + 1) & ~1;
+  const int ns = padded_sources(n, kPW32 * F);
   const size_t rpc = (size_t)(32 / F) * 4;
   return (size_t)40 * ns + ((size_t)kPW32 + 2 * (size_t)rounds) * rpc * 3 * sizeof(double);
 }
@@ -527,7 +545,17 @@ const void* persist_fn_f(int W, bool excl) {
   return nullptr;
 }
 
+// The widths between the forced ones (16 warps only).
+template <int F, int NI>
+const void* persist_fn_16(int W, bool excl) {
+  if (W != 16) return nullptr;
+  return excl ? (const void*)k_run_small_f64<F, 16, NI, true> : (const void*)k_run_small_f64<F, 16, NI, false>;
+}
+
 const void* persist_fn(int F, int W, int NI, bool excl) {
+  if (NI == 5) return F == 16 ? persist_fn_16<16, 5>(W, excl) : F == 8 ? persist_fn_16<8, 5>(W, excl) : nullptr;
+  if (NI == 6) return F == 16 ? persist_fn_16<16, 6>(W, excl) : F == 8 ? persist_fn_16<8, 6>(W, excl) : nullptr;
+  if (NI == 7) return F == 16 ? persist_fn_16<16, 7>(W, excl) : F == 8 ? persist_fn_16<8, 7>(W, excl) : nullptr;
   if (NI == 4) {
     switch (F) {
       case 4: return persist_fn_f<4, 4>(W, excl);
@@ -549,7 +577,7 @@ const void* persist_fn(int F, int W, int NI, bool excl) {
 // Shared memory of a launch: positions and masses, the warps' partial sums, and
 // the velocities of up to `rounds` receiver chunks per CTA.
 size_t persist_smem(int n, int F, int W, int NI, int rounds) {
-  const int ns = (n + 1) & ~1;
+  const int ns = padded_sources(n, W * F);
   const size_t rpc = (size_t)(32 / F) * NI;
   return (size_t)4 * ns * sizeof(double) + ((size_t)W + rounds) * rpc * 3 * sizeof(double);
 }
@@ -562,6 +590,21 @@ int persist_groups(int n, int sms) {
   for (int F : {16, 8, 4})
     if ((32 / F) * kPNIDefault >= need) return F;
   return 4;
+}
+// FP64: the layout with the fewest slots that holds them, among 8 or 16 lane
+// groups of 4 to 7 receivers per lane and the one above: the pair loop runs
+// over the slots, used or not (N = 2048 has 14 receivers per CTA: 14 slots, not
+// 16; N = 3000 21 of 24, not 32: 17.2 -> 14.0 us per step).
+void persist_layout64(int n, int sms, int* F, int* NI) {
+  const int need = (n + sms - 1) / sms;
+  *F = persist_groups(n, sms);
+  *NI = kPNIDefault;
+  for (int f : {16, 8})
+    for (int ni : {4, 5, 6, 7})
+      if ((32 / f) * ni >= need && (32 / f) * ni < (32 / *F) * *NI) {
+        *F = f;
+        *NI = ni;
+      }
 }
 
 }  // namespace
@@ -612,8 +655,10 @@ int run_persistent(nbr_ctx* c, int precision, int scheme, double dt, size_t step
 
   const ForceConfig& o = c->override_cfg[precision];
   int F = persist_groups(n, c->sms), W = kPersistDefaultWarps, NI = kPNIDefault;
+  if (precision == kFP64) persist_layout64(n, c->sms, &F, &NI);
   if (o.ni == kPersistNI) {
     F = o.warps;
+    NI = kPNIDefault;
     if (o.split > 1) W = o.split;
     if (o.tile > 0) NI = o.tile;
   }

@@ -159,3 +159,19 @@ def test_persistent_fp32c_far_from_the_origin(ctx, nbr, oracle):
         assert np.abs(got[k] - want[k]).max() <= 1e-6, k
     for k in ("x", "y", "z"):
         assert np.abs(got[k] - want[k]).max() <= 1e-6 * (1.0 + np.abs(want[k]).max()), k
+
+
+# One size per default layout of the FP64 launch (slots per chunk of n / 148
+# receivers) and per padding of its sources: whole, one short, one over.
+@pytest.mark.parametrize("eps2", [0.0, 1e-4])
+@pytest.mark.parametrize("n", [2, 3, 255, 256, 257, 1184, 1185, 1400, 1600, 1999, 2048, 2049, 2500,
+                               3200, 3800, 4095, 4096])
+def test_persistent_layouts(ctx, nbr, oracle, n, eps2):
+    s = nbr.plummer(n, n)
+    want = oracle.kdk(s, 1e-4, 3, eps2=eps2)
+    for prec, tol in ((0, 1e-11), (1, 1e-6)):
+        ctx.upload(s)
+        assert ctx.run(prec, nbr.KDK, 2, 1e-4, 3, eps2=eps2)["kernels"] == 1
+        got = ctx.download()
+        for k in ("x", "y", "z", "vx", "vy", "vz"):
+            assert np.abs(got[k] - want[k]).max() <= tol, (prec, k)
