@@ -934,6 +934,31 @@ __global__ void __launch_bounds__(128) k_batch_n3_reduce(const BatchParams p, co
   }
 }
 
+// The state without the systems' padding: one warp per tile copies its real
+// particles of the six arrays to their caller's places.
+struct BatchRows {
+  const double* src[6];
+};
+__global__ void __launch_bounds__(128)
+    k_batch_flatten(const BatchRows rows, double* dst, long long n_real, const long long* poff,
+                    const long long* off, int nsys, long long ntiles) {
+  const int lane = threadIdx.x & 31;
+  const long long tile = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (tile >= ntiles) return;
+  const long long first = tile * kTile;
+  int lo = 0, hi = nsys;  // the last system that begins at or before the tile
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) / 2;
+    if (poff[mid] <= first) lo = mid;
+    else hi = mid;
+  }
+  const long long to = off[lo] + (first - poff[lo]);
+  const int count = (int)min((long long)kTile, off[lo + 1] - to);
+#pragma unroll
+  for (int f = 0; f < 6; ++f)
+    for (int k = lane; k < count; k += 32) dst[f * n_real + to + k] = rows.src[f][first + k];
+}
+
 // Per-system diagnostics: one CTA per system.  out[s * 9 + c] =
 // T, Px, Py, Pz, Lx, Ly, Lz, M, U (softened, FP64, fixed-order reductions).
 __global__ void __launch_bounds__(256)
@@ -1167,6 +1192,8 @@ void nbr::BatchState::release() {
   s.release();
   dfree(d_poff);
   dfree(d_nreal);
+  dfree(d_off);
+  dfree(d_flat);
   dfree(d_sys_of_tile);
   dfree(d_items[0]);
   dfree(d_items[1]);
@@ -1316,6 +1343,11 @@ int nbr_batch_upload(nbr_ctx* c, size_t nsys, const size_t* offsets, const doubl
   }
   e = dalloc((void**)&b.d_poff, (nsys + 1) * sizeof(long long));
   if (e == cudaSuccess) e = dalloc((void**)&b.d_nreal, nsys * sizeof(int));
+  const std::vector<long long> off(offsets, offsets + nsys + 1);
+  if (e == cudaSuccess) e = dalloc((void**)&b.d_off, (nsys + 1) * sizeof(long long));
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(b.d_off, off.data(), (nsys + 1) * sizeof(long long), cudaMemcpyHostToDevice,
+                        c->stream);
   for (int wl = 0; wl < 4 && e == cudaSuccess; ++wl)
     e = dalloc((void**)dl[wl], lists[wl].size() * sizeof(int2));
   for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
@@ -1358,19 +1390,21 @@ int nbr_batch_download(nbr_ctx* c, double* x, double* y, double* z, double* vx, 
   BatchState& b = c->bat;
   if (b.nsys == 0) return fail(c, NBR_ERR_NO_SYSTEM, "no batch uploaded");
   cudaSetDevice(c->device);
-  std::vector<double> h(b.s.n_pad);
   cudaError_t e = cudaSuccess;
-  auto get = [&](double* dst, const double* d) {
-    if (!dst || e != cudaSuccess) return;
-    e = cudaMemcpyAsync(h.data(), d, b.s.n_pad * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    if (e != cudaSuccess) return;
-    for (size_t s = 0; s < b.nsys; ++s)
-      std::memcpy(dst + b.off[s], &h[b.poff[s]], (b.off[s + 1] - b.off[s]) * sizeof(double));
-  };
+  if (!b.d_flat) e = dalloc((void**)&b.d_flat, 6 * b.n_real * sizeof(double));
+  if (e != cudaSuccess) return cuda_fail(c, e, "batch download buffer");
   const int a = b.s.cur;
-  get(x, b.s.pos[a][0]); get(y, b.s.pos[a][1]); get(z, b.s.pos[a][2]);
-  get(vx, b.s.vel[0]); get(vy, b.s.vel[1]); get(vz, b.s.vel[2]);
+  const BatchRows rows{{b.s.pos[a][0], b.s.pos[a][1], b.s.pos[a][2], b.s.vel[0], b.s.vel[1], b.s.vel[2]}};
+  const long long ntiles = b.poff[b.nsys] / kTile;
+  k_batch_flatten<<<(unsigned)((ntiles + 3) / 4), 128, 0, c->stream>>>(
+      rows, b.d_flat, (long long)b.n_real, b.d_poff, b.d_off, (int)b.nsys, ntiles);
+  e = cudaGetLastError();
+  double* out[6] = {x, y, z, vx, vy, vz};
+  for (int f = 0; f < 6; ++f)
+    if (out[f] && e == cudaSuccess)
+      e = cudaMemcpyAsync(out[f], b.d_flat + f * b.n_real, b.n_real * sizeof(double),
+                          cudaMemcpyDeviceToHost, c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   return e == cudaSuccess ? NBR_OK : cuda_fail(c, e, "batch download");
 }
 

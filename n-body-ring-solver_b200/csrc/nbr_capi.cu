@@ -490,6 +490,47 @@ int check_device_error(nbr_ctx* c) {
   cudaError_t e = cudaMemcpyAsync(&h, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "kernel execution");
+  return device_error_status(c, h);
+}
+
+cudaError_t stage_fetch(nbr_ctx* c, const StageArrays& a, double* dst, int words[2]) {
+  size_t total = 0;
+  for (int k = 0; k < a.count; ++k) total += (size_t)a.n[k];
+  c->h_stage.resize(std::max(c->h_stage.size(), total + 1));
+  cudaError_t e = launch_stage_out(a, dst, c->d_err, c->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(c->h_stage.data(), dst, (total + 1) * sizeof(double),
+                        cudaMemcpyDeviceToHost, c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  if (e == cudaSuccess) std::memcpy(words, c->h_stage.data() + total, 2 * sizeof(int));
+  return e;
+}
+
+cudaError_t stage_download(nbr_ctx* c, int count, const double* const* src, double* const* out,
+                           size_t n, int* err, int* flags) {
+  StageArrays a{};
+  double* to[8];
+  for (int k = 0; k < count; ++k) {
+    if (!out[k]) continue;
+    a.dev[a.count] = const_cast<double*>(src[k]);
+    a.n[a.count] = (long long)n;
+    to[a.count++] = out[k];
+  }
+  const int arrays = a.count;
+  if (a.count == 0) a.count = 1;  // the error words alone
+  cudaError_t e = c->scr.need_red(arrays * n + 2);
+  int words[2] = {0, 0};
+  if (e == cudaSuccess) e = stage_fetch(c, a, c->scr.red, words);
+  if (e != cudaSuccess) return e;
+  *err = words[0];
+  if (flags) *flags = words[1];
+  if (*err == kErrNone && !(flags && *flags))
+    for (int k = 0; k < arrays; ++k)
+      std::memcpy(to[k], c->h_stage.data() + (size_t)k * n, n * sizeof(double));
+  return cudaSuccess;
+}
+
+int device_error_status(nbr_ctx* c, int h) {
   if (h != kErrNone) {
     cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
     if (c->scr.cnt) cudaMemsetAsync(c->scr.cnt, 0, c->scr.cnt_cap * sizeof(unsigned), c->stream);
@@ -698,9 +739,10 @@ int diag_system(nbr_ctx* c, double G, double eps2, nbr_diag* out) {
   SysState& s = c->sys;
   const int a = s.cur;
   const int nb = (int)((s.n + 127) / 128);
-  // moments (8 x nb), their sums (16), then the potential's sums and U: sized
-  // once here so that nothing below reallocates.
-  cudaError_t e = c->scr.need_red((size_t)nb * 9 + 32 + potential_sums(c));
+  // moments (8 x nb), their sums (16), then the potential's sums and U, then
+  // the results packed: sized once here so that nothing below reallocates.
+  const size_t used = (size_t)nb * 9 + 32 + potential_sums(c);
+  cudaError_t e = c->scr.need_red(used + 16);
   if (e != cudaSuccess) return cuda_fail(c, e, "diag scratch");
   double* part = c->scr.red;
   double* res = c->scr.red + (size_t)nb * 8;
@@ -711,14 +753,16 @@ int diag_system(nbr_ctx* c, double G, double eps2, nbr_diag* out) {
   double *dU = nullptr, factor = 1.0;
   int rc = potential_system(c, G, eps2, nullptr, (size_t)nb * 9 + 16, &dU, &factor);
   if (rc) return rc;
-  double h[9];
-  e = cudaMemcpyAsync(h, res, 8 * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(h + 8, dU, sizeof(double), cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  StageArrays sa{};
+  sa.count = 2;
+  sa.dev[0] = res; sa.n[0] = 8;
+  sa.dev[1] = dU; sa.n[1] = 1;
+  int words[2];
+  e = stage_fetch(c, sa, c->scr.red + used, words);
   if (e != cudaSuccess) return cuda_fail(c, e, "diagnostics");
-  rc = check_device_error(c);
+  rc = device_error_status(c, words[0]);
   if (rc) return rc;
+  const double* h = c->h_stage.data();
   out->T = h[0];
   out->P[0] = h[1]; out->P[1] = h[2]; out->P[2] = h[3];
   out->L[0] = h[4]; out->L[1] = h[5]; out->L[2] = h[6];
@@ -815,7 +859,7 @@ int nbr_ctx_destroy(nbr_ctx* c) {
   if (!c) return NBR_OK;
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  c->run_graph.release();
+  for (RunGraph& g : c->run_graph) g.release();
   c->sys.release();
   c->bat.release();
   c->scr.release();
@@ -852,7 +896,10 @@ int nbr_system_upload(nbr_ctx* c, size_t n, const double* x, const double* y, co
   if (n > (size_t)1 << 31) return fail(c, NBR_ERR_INVALID_ARG, "n above 2^31");
   cudaSetDevice(c->device);
   SysState& s = c->sys;
+  const size_t cap0 = s.cap;
   cudaError_t e = s.reserve(n);
+  if (s.cap != cap0)  // their buffers are gone
+    for (RunGraph& g : c->run_graph) g.release();
   if (e != cudaSuccess) return cuda_fail(c, e, "system allocation");
   s.cur = 0;
   s.rec_ok[0] = s.rec_ok[1] = false;
@@ -901,6 +948,15 @@ int nbr_system_download(nbr_ctx* c, double* x, double* y, double* z, double* vx,
   cudaSetDevice(c->device);
   const size_t B = s.n * sizeof(double);
   cudaError_t e = cudaSuccess;
+  if (stage_fits(6 * s.n)) {
+    const double* src[6] = {s.pos[s.cur][0], s.pos[s.cur][1], s.pos[s.cur][2],
+                            s.vel[0], s.vel[1], s.vel[2]};
+    double* out[6] = {x, y, z, vx, vy, vz};
+    int err = 0;
+    e = stage_download(c, 6, src, out, s.n, &err);
+    if (e != cudaSuccess) return cuda_fail(c, e, "download");
+    return device_error_status(c, err);
+  }
   auto D = [&](double* h, const double* d) {
     if (h && e == cudaSuccess) e = cudaMemcpyAsync(h, d, B, cudaMemcpyDeviceToHost, c->stream);
   };
@@ -923,12 +979,23 @@ int nbr_forces(nbr_ctx* c, int precision, double G, double eps2, int want_force,
   cudaSetDevice(c->device);
   int rc = eval_system(c, precision, G, eps2, 0, 0.0, 0.0, want_force, nullptr);
   if (rc) return rc;
-  rc = check_device_error(c);
+  const bool staged = stage_fits(3 * s.n);
+  if (staged) {
+    const double* src[3] = {s.acc[0], s.acc[1], s.acc[2]};
+    double* out[3] = {ax, ay, az};
+    int err = 0;
+    const cudaError_t e = stage_download(c, 3, src, out, s.n, &err);
+    if (e != cudaSuccess) return cuda_fail(c, e, "kernel execution");
+    rc = device_error_status(c, err);
+  } else {
+    rc = check_device_error(c);
+  }
   if (rc) return rc;
   c->acc_ok = !want_force;
   c->acc_prec = precision;
   c->acc_G = G;
   c->acc_eps2 = eps2;
+  if (staged) return NBR_OK;
   const size_t B = s.n * sizeof(double);
   cudaError_t e = cudaSuccess;
   auto D = [&](double* h, const double* d) {
@@ -1136,9 +1203,12 @@ int nbr_accel_ij(nbr_ctx* c, int precision, size_t n_i, const double* xi, const 
   if (!(eps2 >= 0.0) || !std::isfinite(eps2) || !std::isfinite(G))
     return fail(c, NBR_ERR_INVALID_ARG, "eps2 must be finite and >= 0, G finite");
   if (n_i > (size_t)1 << 31 || n_j > (size_t)1 << 31) return fail(c, NBR_ERR_INVALID_ARG, "size above 2^31");
-  if (!finite_array(xi, n_i) || !finite_array(yi, n_i) || !finite_array(zi, n_i) ||
-      (mi && !finite_array(mi, n_i)) || !finite_array(xj, n_j) || !finite_array(yj, n_j) ||
-      !finite_array(zj, n_j) || !finite_array(mj, n_j))
+  // small sets: one transfer each way, the check on the device
+  const bool staged = n_j > 0 && stage_fits((mi ? 4 : 3) * n_i + 4 * n_j);
+  if (!staged &&
+      (!finite_array(xi, n_i) || !finite_array(yi, n_i) || !finite_array(zi, n_i) ||
+       (mi && !finite_array(mi, n_i)) || !finite_array(xj, n_j) || !finite_array(yj, n_j) ||
+       !finite_array(zj, n_j) || !finite_array(mj, n_j)))
     return fail(c, NBR_ERR_NONFINITE, "input contains NaN or Inf");
   if (n_j == 0) {
     std::fill(ax, ax + n_i, 0.0); std::fill(ay, ay + n_i, 0.0); std::fill(az, az + n_i, 0.0);
@@ -1157,10 +1227,35 @@ int nbr_accel_ij(nbr_ctx* c, int precision, size_t n_i, const double* xi, const 
     if (e == cudaSuccess && (long long)n < np)
       e = cudaMemsetAsync(d + n, 0, (np - n) * sizeof(double), c->stream);
   };
-  H(r.pos[0][0], xi, n_i, npi); H(r.pos[0][1], yi, n_i, npi); H(r.pos[0][2], zi, n_i, npi);
-  if (mi) H(r.mass, mi, n_i, npi);
-  H(r.pos[1][0], xj, n_j, npj); H(r.pos[1][1], yj, n_j, npj); H(r.pos[1][2], zj, n_j, npj);
-  H(r.vel[0], mj, n_j, npj);  // source masses
+  if (staged) {
+    StageArrays sa{};
+    size_t off = 0;
+    const size_t total = (mi ? 4 : 3) * n_i + 4 * n_j;
+    c->h_stage.resize(std::max(c->h_stage.size(), total));
+    e = c->scr.need_red(total);
+    if (e != cudaSuccess) return cuda_fail(c, e, "ij staging");
+    auto put = [&](double* d, const double* h, size_t n, long long np) {
+      if (!h) return;
+      std::memcpy(c->h_stage.data() + off, h, n * sizeof(double));
+      off += n;
+      sa.dev[sa.count] = d;
+      sa.n[sa.count] = (long long)n;
+      sa.n_pad[sa.count++] = np;
+    };
+    put(r.pos[0][0], xi, n_i, npi); put(r.pos[0][1], yi, n_i, npi); put(r.pos[0][2], zi, n_i, npi);
+    put(r.mass, mi, n_i, npi);
+    put(r.pos[1][0], xj, n_j, npj); put(r.pos[1][1], yj, n_j, npj); put(r.pos[1][2], zj, n_j, npj);
+    put(r.vel[0], mj, n_j, npj);  // source masses
+    e = cudaMemcpyAsync(c->scr.red, c->h_stage.data(), total * sizeof(double),
+                        cudaMemcpyHostToDevice, c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->d_err + 1, 0, sizeof(int), c->stream);
+    if (e == cudaSuccess) e = launch_stage_in(sa, c->scr.red, c->d_err + 1, c->stream);
+  } else {
+    H(r.pos[0][0], xi, n_i, npi); H(r.pos[0][1], yi, n_i, npi); H(r.pos[0][2], zi, n_i, npi);
+    if (mi) H(r.mass, mi, n_i, npi);
+    H(r.pos[1][0], xj, n_j, npj); H(r.pos[1][1], yj, n_j, npj); H(r.pos[1][2], zj, n_j, npj);
+    H(r.vel[0], mj, n_j, npj);  // source masses
+  }
   if (e != cudaSuccess) return cuda_fail(c, e, "ij upload");
   const int ntiles = (int)((n_j + kTile - 1) / kTile);
   if (precision == kFP32C) {
@@ -1191,6 +1286,16 @@ int nbr_accel_ij(nbr_ctx* c, int precision, size_t n_i, const double* xi, const 
       ep.part_len = (long long)c->scr.part_cap; ep.cnt_len = (long long)c->scr.cnt_cap;)
   e = launch_force(precision, eps2, cfg, ip, js, ep, c->stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "ij force launch");
+  if (staged) {
+    const double* src[3] = {r.acc[0], r.acc[1], r.acc[2]};
+    double* out[3] = {ax, ay, az};
+    int err = 0, flags = 0;
+    e = stage_download(c, 3, src, out, n_i, &err, &flags);
+    if (e != cudaSuccess) return cuda_fail(c, e, "kernel execution");
+    rc = device_error_status(c, err);
+    if (rc) return rc;
+    return flags ? fail(c, NBR_ERR_NONFINITE, "input contains NaN or Inf") : NBR_OK;
+  }
   rc = check_device_error(c);
   if (rc) return rc;
   const size_t B = n_i * sizeof(double);
@@ -1300,7 +1405,11 @@ int nbr_run(nbr_ctx* c, int precision, int scheme, int order, double dt, size_t 
     key.ptr[0] = s.pos[0][0]; key.ptr[1] = s.rec[0]; key.ptr[2] = s.vel[0];
     key.ptr[3] = c->scr.part; key.ptr[4] = c->scr.cnt; key.ptr[5] = c->d_err;
     key.ptr[6] = c->n3_order;
-    RunGraph& rg = c->run_graph;
+    // the matching graph to the front; none: the oldest makes room
+    int at = 0;
+    while (at < kRunGraphs - 1 && !(c->run_graph[at].exec && c->run_graph[at].key == key)) ++at;
+    std::rotate(c->run_graph, c->run_graph + at, c->run_graph + at + 1);
+    RunGraph& rg = c->run_graph[0];
     int kernels = 0;
     double evals = 0;
     cudaError_t e = cudaSuccess;
@@ -1379,14 +1488,17 @@ int nbr_run(nbr_ctx* c, int precision, int scheme, int order, double dt, size_t 
     e = cudaEventRecord(c->ev0, c->stream);
     if (e == cudaSuccess) e = cudaGraphLaunch(rg.exec, c->stream);
     if (e == cudaSuccess) e = cudaEventRecord(c->ev1, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
       rg.release();
       c->acc_ok = false;
       return cuda_fail(c, e, "graph launch");
     }
-    rc = check_device_error(c);
-    if (rc) return rc;
+    rc = check_device_error(c);  // waits for the stream
+    if (rc) {
+      if (rc == NBR_ERR_CUDA) rg.release();
+      c->acc_ok = false;
+      return rc;
+    }
     float ms = 0.f;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
     st.gpu_ms = ms;

@@ -64,6 +64,8 @@ struct BatchState {
   std::vector<long long> poff;       // padded offsets (host), nsys + 1
   long long* d_poff = nullptr;       // padded offsets (device), nsys + 1
   int* d_nreal = nullptr;            // real size of each system (device)
+  long long* d_off = nullptr;        // real offsets (device), nsys + 1
+  double* d_flat = nullptr;          // [6][n_real]: the state without padding (first download)
   int* d_sys_of_tile = nullptr;      // system index of every padded tile
   // Work queues of (system | kWideItem flag, first receiver tile), cost
   // ordered: [0] one-tile items only, [1] two-tile items where a system has
@@ -125,6 +127,20 @@ cudaError_t dalloc(void** p, size_t bytes);
 void dfree(void* p);
 bool finite_array(const double* a, size_t n);
 int check_device_error(nbr_ctx* c);
+// The status of a device error word already on the host (0: NBR_OK).
+int device_error_status(nbr_ctx* c, int h);
+// Arrays of up to kStageBytes in all travel between the host and the device in
+// one transfer, packed in Scratch::red on the device and in nbr_ctx::h_stage on
+// the host.
+constexpr size_t kStageBytes = 1 << 20;
+inline bool stage_fits(size_t doubles) { return doubles * sizeof(double) <= kStageBytes; }
+// The arrays of a, packed at dst (device scratch), into c->h_stage, and the
+// device error block's first two words into words; waits for the stream.
+cudaError_t stage_fetch(nbr_ctx* c, const StageArrays& a, double* dst, int words[2]);
+// count arrays of n doubles each into out[k] (null: left out), unless *err (the
+// device error word) or *flags (the input flags) is set.
+cudaError_t stage_download(nbr_ctx* c, int count, const double* const* src, double* const* out,
+                           size_t n, int* err, int* flags = nullptr);
 // Bounded-wait limit and tile-skip test hook from the environment.
 void pipeline_params(JStream& js);
 // The persistent small-system run (nbr_persist.cu): whether it serves an
@@ -153,7 +169,8 @@ struct RunKey {
   const void* ptr[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   bool operator==(const RunKey& o) const;
 };
-// The last nbr_run graph, replayed while the key matches.
+// A captured nbr_run graph, replayed while the key matches.
+constexpr int kRunGraphs = 4;
 struct RunGraph {
   cudaGraphExec_t exec = nullptr;
   RunKey key;
@@ -183,7 +200,16 @@ struct nbr_ctx {
   int acc_prec = 0;
   double acc_G = 0.0, acc_eps2 = 0.0;
   nbr::ForceConfig override_cfg[2] = {{0, 0, 0}, {0, 0, 0}};
-  nbr::RunGraph run_graph;
+  // The last graphs of nbr_run, most recent first: a run of an odd number of
+  // position updates ends in the other buffer, so a repeated call alternates
+  // between two.
+  nbr::RunGraph run_graph[nbr::kRunGraphs];
+  std::vector<double> h_stage;
+  // The last persistent launch configuration whose attributes were set, and its
+  // resident CTAs per SM.
+  const void* persist_fn = nullptr;
+  size_t persist_smem = 0;
+  int persist_per_sm = 0;
   // Launch order of the whole-system Newton-3 grid (longest CTA first) for
   // n3_order_nb blocks, then its inverse; written before any graph capture
   // (n3_order_prepare, the only writer), read by the pair and reduce kernels.

@@ -1657,6 +1657,34 @@ __global__ void __launch_bounds__(256) k_validate(long long n, const double* __r
   if ((threadIdx.x & 31) == 0 && f) atomicOr(flags, f);
 }
 
+// ------------------------------------------------------------- staging ----
+// blockIdx.y: the array.  Bound by the launch; one copy follows or precedes it
+// in place of one per array.  Whole calls on B200, before / with it: download of
+// 64 particles 80 / 42 us, of 2048 92 / 67; nbr_accel_ij 8000 x 8000 298 / 251;
+// nbr_diagnostics of 2000 65 / 49.  (Pinned host memory would take another 8 to
+// 45 us off them and 1 to 3 ms to allocate per context.)
+__global__ void __launch_bounds__(256) k_stage_out(const StageArrays a, double* dst,
+                                                   const int* err) {
+  const int k = blockIdx.y;
+  long long off = 0;
+  for (int q = 0; q < k; ++q) off += a.n[q];
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < a.n[k]) dst[off + i] = a.dev[k][i];
+  if (i < 2 && k + 1 == a.count) reinterpret_cast<int*>(dst + off + a.n[k])[i] = err[i];
+}
+
+__global__ void __launch_bounds__(256) k_stage_in(const StageArrays a, const double* __restrict__ src,
+                                                  int* flags) {
+  const int k = blockIdx.y;
+  long long off = 0;
+  for (int q = 0; q < k; ++q) off += a.n[q];
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.n_pad[k]) return;
+  const double v = i < a.n[k] ? src[off + i] : 0.0;
+  a.dev[k][i] = v;
+  if (!isfinite(v)) atomicOr(flags, 1);
+}
+
 // -------------------------------------------------------------- dispatch ----
 #define NBR_CFG_LIST(X) X(4, 2) X(4, 4) X(4, 8) X(8, 2) X(8, 4)
 #define NBR_SMALL_LIST(X) X(2) X(4) X(8)
@@ -2192,6 +2220,20 @@ cudaError_t launch_moments(long long n, long long n_pad, const double* x, const 
 cudaError_t launch_rowsum(const double* part, int nblocks, int width, double* out,
                           cudaStream_t st) {
   k_rowsum<<<1, 256, 0, st>>>(part, nblocks, width, out);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_stage_out(const StageArrays& a, double* dst, const int* err, cudaStream_t st) {
+  long long most = 2;
+  for (int k = 0; k < a.count; ++k) most = std::max(most, a.n[k]);
+  k_stage_out<<<dim3((unsigned)((most + 255) / 256), a.count), 256, 0, st>>>(a, dst, err);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_stage_in(const StageArrays& a, const double* src, int* flags, cudaStream_t st) {
+  long long most = 1;
+  for (int k = 0; k < a.count; ++k) most = std::max(most, a.n_pad[k]);
+  k_stage_in<<<dim3((unsigned)((most + 255) / 256), a.count), 256, 0, st>>>(a, src, flags);
   return cudaGetLastError();
 }
 

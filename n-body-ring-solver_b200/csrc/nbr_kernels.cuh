@@ -332,6 +332,20 @@ cudaError_t launch_rowsum(const double* part, int nblocks, int width, double* ou
 cudaError_t launch_validate(long long n, const double* x, const double* y, const double* z,
                             const double* vx, const double* vy, const double* vz,
                             const double* m, int* flags, int sms, cudaStream_t stream);
+// Up to 8 arrays of one length between their places and a packed buffer.
+struct StageArrays {
+  int count;
+  long long n[8];       // entries of each array
+  long long n_pad[8];   // stage_in: entries written, zeros from n on
+  double* dev[8];
+};
+// dst[sum of n before k + i] = dev[k][i]; the two words of err after them.
+cudaError_t launch_stage_out(const StageArrays& a, double* dst, const int* err,
+                             cudaStream_t stream);
+// dev[k][i] = src[sum of n before k + i] (device memory) with zero padding; bit 0
+// of *flags is set if an entry is NaN or Inf.
+cudaError_t launch_stage_in(const StageArrays& a, const double* src, int* flags,
+                            cudaStream_t stream);
 size_t force_smem_bytes(int precision, const ForceConfig& cfg);
 // Resident CTAs per SM of the force kernel for this configuration (0 on error).
 int force_blocks_per_sm(int precision, double eps2, const ForceConfig& cfg);

@@ -52,7 +52,10 @@ struct PersistArgs {
   int chunks;              // receiver chunks of cs particles
   int cs;                  // receivers per chunk (<= RPC slots of the lane layout)
   int evals;               // force evaluations
-  const double2* sched;    // (kick, drift) of every evaluation
+  // (kick, drift) of the evaluations: the last, the first, and the others by
+  // their place in a step of `period` evaluations
+  double2 last, first, cycle[15];
+  int period;
   int mode;                // 1: leapfrog (drift with the kicked velocity); 2: Euler
   int pre;                 // a standalone kick/drift before the first evaluation
   int pre_use_acc;         // its kick uses the accelerations left by the last run
@@ -234,7 +237,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_run_small_f64(const PersistArgs A
       }
     }
     __syncthreads();
-    const double2 kd = A.sched[e];
+    const double2 kd = e + 1 == A.evals ? A.last : e == 0 ? A.first : A.cycle[e % A.period];
     for (int c = blockIdx.x, round = 0; c < A.chunks; c += gridDim.x, ++round) {
       const int base = c * A.cs;
       double xi[kPNI], yi[kPNI], zi[kPNI], ax[kPNI], ay[kPNI], az[kPNI];
@@ -431,7 +434,7 @@ __global__ void __launch_bounds__(kPW32 * 32, 1) k_run_small_f32c(const PersistA
       }
     }
     __syncthreads();
-    const double2 kd = A.sched[e];
+    const double2 kd = e + 1 == A.evals ? A.last : e == 0 ? A.first : A.cycle[e % A.period];
     for (int c = blockIdx.x, round = 0; c < A.chunks; c += gridDim.x, ++round) {
       const int base = c * A.cs;
       double* sp = spos + (size_t)round * RPC * 3;
@@ -620,34 +623,35 @@ int run_persistent(nbr_ctx* c, int precision, int scheme, double dt, size_t step
                    nbr_run_stats* st) {
   SysState& s = c->sys;
   const int n = (int)s.n;
-  // the schedule: the launch sequence of nbr_run's graph, one entry per evaluation
-  std::vector<double2> sched;
+  // the schedule: the launch sequence of nbr_run's graph
   PersistArgs A{};
+  size_t evals = steps;
+  A.period = 1;
   A.mode = scheme == NBR_EULER ? 2 : 1;
   if (scheme == NBR_KDK) {
     if (fsal) {
       A.pre = 1; A.pre_use_acc = 1; A.pre_kick = 0.5 * dt; A.pre_drift = dt;
     } else {
-      sched.push_back(make_double2(0.5 * dt, dt));
+      evals += 1;
     }
-    for (size_t k = 1; k < steps; ++k) sched.push_back(make_double2(dt, dt));
-    sched.push_back(make_double2(0.5 * dt, 0.0));
+    A.cycle[0] = make_double2(dt, dt);
+    A.first = fsal ? A.cycle[0] : make_double2(0.5 * dt, dt);
+    A.last = make_double2(0.5 * dt, 0.0);
   } else if (scheme == NBR_EULER) {
-    for (size_t k = 0; k < steps; ++k) sched.push_back(make_double2(dt, dt));
+    A.first = A.last = A.cycle[0] = make_double2(dt, dt);
   } else {
     A.pre = 1; A.pre_use_acc = 0; A.pre_kick = 0.0; A.pre_drift = cc[0] * dt;
-    for (size_t k = 0; k < steps; ++k)
-      for (int sub = 0; sub < lf - 1; ++sub) {
-        const double drift = sub < lf - 2 ? cc[sub + 1]
-                                          : ((k + 1 < steps) ? cc[lf - 1] + cc[0] : cc[lf - 1]);
-        sched.push_back(make_double2(dd[sub] * dt, drift * dt));
-      }
+    A.period = lf - 1;
+    evals = steps * (size_t)(lf - 1);
+    for (int sub = 0; sub < lf - 1; ++sub)
+      A.cycle[sub] = make_double2(
+          dd[sub] * dt, (sub < lf - 2 ? cc[sub + 1] : cc[lf - 1] + cc[0]) * dt);
+    A.first = A.cycle[0];
+    A.last = make_double2(dd[lf - 2] * dt, cc[lf - 1] * dt);
   }
-  const int E = (int)sched.size();
-  cudaError_t e = c->scr.need_red((size_t)2 * E + 16);
-  if (e != cudaSuccess) return cuda_fail(c, e, "persistent schedule");
-  e = cudaMemcpyAsync(c->scr.red, sched.data(), sched.size() * sizeof(double2),
-                      cudaMemcpyHostToDevice, c->stream);
+  if (evals > 0x7fffffff) return fail(c, NBR_ERR_INVALID_ARG, "too many steps in one run");
+  const int E = (int)evals;
+  cudaError_t e = cudaSuccess;
   // the arrival counter: the context's error block words 2-3 (8-byte aligned)
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(c->d_err + 2);
   if (e == cudaSuccess) e = cudaMemsetAsync(bar, 0, sizeof(unsigned long long), c->stream);
@@ -681,17 +685,20 @@ int run_persistent(nbr_ctx* c, int precision, int scheme, double dt, size_t step
   // the grid is at least min(chunks, SMs) CTAs, so no CTA gets more rounds than this
   const int rounds = (chunks + std::min(chunks, c->sms) - 1) / std::min(chunks, c->sms);
   const size_t smem = fp32 ? persist_smem32(n, F, rounds) : persist_smem(n, F, W, NI, rounds);
+  // (kernel attributes are the process's, so only the occupancy is kept)
   e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  int per_sm = 0;
-  if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kPThreads, smem);
+  if (e == cudaSuccess && (fn != c->persist_fn || smem != c->persist_smem)) {
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->persist_per_sm, fn, kPThreads, smem);
+    c->persist_fn = e == cudaSuccess ? fn : nullptr;
+    c->persist_smem = smem;
+  }
   if (e != cudaSuccess) return cuda_fail(c, e, "persistent kernel setup");
+  const int per_sm = c->persist_per_sm;
   if (per_sm < 1) return fail(c, NBR_ERR_UNSUPPORTED, "persistent kernel does not fit an SM");
   A.n = n;
   A.chunks = chunks;
   A.cs = cs;
   A.evals = E;
-  A.sched = reinterpret_cast<const double2*>(c->scr.red);
   A.G = G;
   A.eps2 = eps2;
   for (int b = 0; b < 2; ++b) {
@@ -713,14 +720,13 @@ int run_persistent(nbr_ctx* c, int precision, int scheme, double dt, size_t step
   if (e == cudaSuccess)
     e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kPThreads), args, smem, c->stream);
   if (e == cudaSuccess) e = cudaEventRecord(c->ev1, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) {
     c->acc_ok = false;
     return cuda_fail(c, e, "persistent run launch");
   }
   s.cur = (s.cur + A.pre + E) & 1;
   s.rec_ok[0] = s.rec_ok[1] = false;
-  const int rc = check_device_error(c);
+  const int rc = check_device_error(c);  // waits for the stream
   if (rc) return rc;
   float ms = 0.f;
   cudaEventElapsedTime(&ms, c->ev0, c->ev1);
