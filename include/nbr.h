@@ -402,7 +402,8 @@ int nbr_batch_run(nbr_ctx* ctx, int precision, double dt, size_t steps, double G
  * tiles, each pair once: FP32C two-tile blocks for systems of three tiles
  * (257 particles) or more, the others as for wide = 1; FP64 one-tile blocks
  * for systems of two tiles (129 particles) or more, the others as for
- * wide = 0; ctas_per_sm = resident CTAs per SM of the persistent grid (0: the
+ * wide = 0; ctas_per_sm = resident CTAs per SM of the persistent grid (0: for
+ * wide = 2 the count a model of the batch finishes first with, else the
  * occupancy limit).  wide = -1 restores the autotune cache or the default
  * (occupancy limit; Newton-3 row blocks).  Applies to the uploaded batch; an
  * upload starts from the autotune cache again.  The Newton-3 scratch (3

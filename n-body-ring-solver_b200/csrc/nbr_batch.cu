@@ -639,8 +639,10 @@ __device__ __forceinline__ bool run_item_n3(const BatchParams& p, u64 EPS2, Ring
 // lane (lane + 32 k) -- against the system's column tiles c >= r.  Its own
 // tile: every ordered pair, action only (tile_f64).  Each later tile c: every
 // pair once, the tile's sources in batches of 32, one per lane, rotating
-// through the warp by shuffles with their reaction sums (the scheme of
-// k_force_n3_f64); batches of padding are skipped.  The reaction of tile c
+// through the warp with their reaction sums: lane l takes source (l - step) mod
+// 32 from the tile in shared memory, one step ahead, and shuffles the reaction
+// sums (1000 systems: 2068 us per step with the sources shuffled too, 1951);
+// batches of padding are skipped.  The reaction of tile c
 // goes to its slot, the action to p.act; the epilogue runs in
 // k_batch_n3_reduce.  Returns false if a tile wait gave up.
 template <bool EXCL>
@@ -718,6 +720,8 @@ __device__ __forceinline__ bool run_item_n3_f64(const BatchParams& p, double eps
         double RX = 0.0, RY = 0.0, RZ = 0.0;
 #pragma unroll 2
         for (int step = 0; step < 32; ++step) {
+          const int jn = bt * 32 + ((lane - step - 1) & 31);  // the next step's source
+          const double nx = SX[jn], ny = SY[jn], nz = SZ[jn], nm = SM[jn];
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             const double dx = sx - xi[k], dy = sy - yi[k], dz = sz - zi[k];
@@ -735,13 +739,10 @@ __device__ __forceinline__ bool run_item_n3_f64(const BatchParams& p, double eps
             RY = fma(si, dy, RY);
             RZ = fma(si, dz, RZ);
           }
-          sx = __shfl_sync(0xffffffffu, sx, from);
-          sy = __shfl_sync(0xffffffffu, sy, from);
-          sz = __shfl_sync(0xffffffffu, sz, from);
-          sm = __shfl_sync(0xffffffffu, sm, from);
           RX = __shfl_sync(0xffffffffu, RX, from);
           RY = __shfl_sync(0xffffffffu, RY, from);
           RZ = __shfl_sync(0xffffffffu, RZ, from);
+          sx = nx; sy = ny; sz = nz; sm = nm;
         }
         // back at its own lane: the acceleration of source j is -sum m_i y^3 d
         if (in) {
@@ -1089,10 +1090,37 @@ void batch_config(nbr_ctx* c, int prec, double eps2) {
   b.cfg_ok[pi] = true;
 }
 
+// Resident CTAs per SM of a Newton-3 work list where none are configured.  A
+// warp's items are one chain each, and warps that share a scheduler slow each
+// other down: with k CTAs per SM an item takes 1 / speed(k) times as long as
+// alone, while the SM does k speed(k) times as much.  A large batch is bound by
+// its total work (the most CTAs), a small one by its largest item (few).
+// speed() is measured on 4096 systems, whose time is total work; the choice it
+// makes agrees with the measured best for every batch below, us per step with
+// the occupancy limit / with the choice: FP64 16 systems of 64 .. 4096 1098 /
+// 967, 200 1619 / 1181, 500 1772 / 1402, 1000 2022 / 2022; FP32C 16 557 / 450, 200 817 /
+// 554, 500 885 / 598, 1000 997 / 997; 1000 of 64 .. 512 FP64 236 / 177, FP32C 114 / 73.
+int batch_ctas_per_sm(const BatchState::N3List& l, int prec, int occ, int sms) {
+  static const double speed64[] = {1.0, 0.870, 0.735, 0.608}, speed32[] = {1.0, 0.641};
+  const double* speed = prec == kFP32C ? speed32 : speed64;
+  const int known = prec == kFP32C ? 2 : 4;
+  int best = occ;
+  double best_t = 0.0;
+  for (int k = std::min(occ, known); k >= 1; --k) {
+    const double v = speed[k - 1];
+    const double t = std::max(l.cost / ((double)sms * kBWarps * k * v), l.cost_max / v);
+    if (best_t == 0.0 || t < best_t) {
+      best_t = t;
+      best = k;
+    }
+  }
+  return best;
+}
+
 // Sets the kernel's shared-memory attribute (once per kernel variant),
 // allocates the Newton-3 scratch at its first use, and returns the
-// persistent grid: resident CTAs per SM (the configured count, at most the
-// occupancy limit) x SMs, or 0 if the scratch allocation failed.  Called
+// persistent grid: resident CTAs per SM (the configured count or
+// batch_ctas_per_sm's, at most the occupancy limit) x SMs, or 0 if the scratch allocation failed.  Called
 // before any stream capture.
 int batch_grid(nbr_ctx* c, int prec, double eps2) {
   BatchState& b = c->bat;
@@ -1120,7 +1148,9 @@ int batch_grid(nbr_ctx* c, int prec, double eps2) {
       per = 1;
     occ = per;
   }
-  const int per = b.per_sm[pi] > 0 ? std::min(b.per_sm[pi], occ) : occ;
+  const int per = b.per_sm[pi] > 0 ? std::min(b.per_sm[pi], occ)
+                  : wi == 2       ? batch_ctas_per_sm(l3, prec, occ, c->sms)
+                                  : occ;
   return per * c->sms;
 }
 
@@ -1326,6 +1356,10 @@ int nbr_batch_upload(nbr_ctx* c, size_t nsys, const size_t* offsets, const doubl
     std::stable_sort(order.begin(), order.end(), [&](int a, int bb) { return cost[a] > cost[bb]; });
     lists[wl].resize(items.size());
     for (size_t k = 0; k < order.size(); ++k) lists[wl][k] = items[order[k]];
+    if (q >= 0) {
+      b.n3[q].cost = std::accumulate(cost.begin(), cost.end(), 0.0);
+      b.n3[q].cost_max = cost.empty() ? 0.0 : cost[order[0]];
+    }
   }
   std::vector<int> nreal(nsys);
   b.max_ns = 0;

@@ -82,6 +82,7 @@ struct BatchState {
   struct N3List {
     int2* d_items = nullptr;
     int n_items = 0;
+    double cost = 0.0, cost_max = 0.0;  // of all items and of the largest one
     int2* d_tiles = nullptr;
     int n_tiles = 0;
     long long* d_rea_off = nullptr;
