@@ -70,6 +70,19 @@ __device__ inline int strip_row(const StripPlan& p, int u) {
   return r;
 }
 
+// The strips and the reduction are launched with programmatic stream
+// serialization: a kernel may be set up while the one before it in the stream
+// finishes.  It reads or writes nothing before grid_dependency_wait(), which
+// returns when that kernel has completed and its writes are visible.  us per
+// evaluation in a graph, without / with: FP64 N = 4224 23.9 / 21.3, 6000 34.7 / 33.6;
+// FP32C 4224 18.4 / 15.4, 6000 22.4 / 21.2, 12001 61.9 / 59.7.
+__device__ __forceinline__ void grid_dependency_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;");
+}
+
 // FP32C.  r^-3 = y^3 (1 - h)^(-3/2) with y the MUFU root and h = 1 - r2 y^2 is
 // y^3 (1 + 3/2 h) to first order = 3/2 y^3 (5/3 - r2 y^2): one fma after y^2, and
 // the masses of both particles multiply it, so a pair costs 3 differences, 3
@@ -101,6 +114,8 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
   extern __shared__ double strip_acc[];  // [kStripWarps][3][32 NI]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = warp * gridDim.x + blockIdx.x;
+  grid_dependency_wait();
+  launch_dependents();
   if (g >= sp.strips) return;
   int u = strip_start(sp, g);
   const int u_end = strip_start(sp, g + 1);
@@ -265,6 +280,8 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
   extern __shared__ double strip_acc[];  // [kStripWarps][3][32 NI]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = warp * gridDim.x + blockIdx.x;
+  grid_dependency_wait();
+  launch_dependents();
   if (g >= sp.strips) return;
   int u = strip_start(sp, g);
   const int u_end = strip_start(sp, g + 1);
@@ -479,6 +496,8 @@ __global__ void __launch_bounds__(32 * kRedWarps)
   const int b = blockIdx.x;                // batch of 32 particles
   const int rb = b / sp.tb;                // its row block
   const long long i = 32LL * b + lane;
+  grid_dependency_wait();
+  launch_dependents();
   if (!NBR_IN(i, ip.len, ep.err)) return;
   double sx = 0.0, sy = 0.0, sz = 0.0;
   if (rb >= sp.r0 && rb < sp.r1) {
@@ -680,16 +699,27 @@ cudaError_t launch_strips(int precision, const StripPlan& p, double eps2, const 
   void* rea = scratch + p.act_doubles;
   int* err = ep.err;
   void* args[] = {&a0, &a1, &a2, precision == kFP32C ? (void*)&e32 : (void*)&e64, &act, &rea, &err};
-  cudaError_t e = cudaLaunchKernel(fn, dim3(sms), dim3(kStripWarps * 32), args,
-                                   strip_smem(p.tb), st);
+  cudaLaunchAttribute serial{};
+  serial.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  serial.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(sms);
+  cfg.blockDim = dim3(kStripWarps * 32);
+  cfg.dynamicSmemBytes = strip_smem(p.tb);
+  cfg.stream = st;
+  cfg.attrs = &serial;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
   if (e != cudaSuccess) return e;
+  cfg.gridDim = dim3(p.batches);
+  cfg.blockDim = dim3(32 * kRedWarps);
+  cfg.dynamicSmemBytes = 0;
+  const void* sums = rea;
   if (precision == kFP32C)
-    k_strip_reduce<kFP32C><<<p.batches, 32 * kRedWarps, 0, st>>>(
-        ip, ep, p, act, rea, 1.0 / ((double)kC53 - 1.0), mode, dst, ld);
-  else
-    k_strip_reduce<kFP64><<<p.batches, 32 * kRedWarps, 0, st>>>(ip, ep, p, act, rea, kInvCubeScale,
-                                                                mode, dst, ld);
-  return cudaGetLastError();
+    return cudaLaunchKernelEx(&cfg, k_strip_reduce<kFP32C>, ip, ep, p, (const double*)act, sums,
+                              1.0 / ((double)kC53 - 1.0), mode, dst, ld);
+  return cudaLaunchKernelEx(&cfg, k_strip_reduce<kFP64>, ip, ep, p, (const double*)act, sums,
+                            kInvCubeScale, mode, dst, ld);
 }
 
 }  // namespace nbr
