@@ -426,7 +426,7 @@ def run_ours(a):
     roofline = {"bound": "fp32_fma_pipe", "achieved": achieved, "peak": peak, "unit": UNIT,
                 "frac": achieved / peak, "traffic": profile_traffic(),
                 "algorithmic_bytes": 96 * n,
-                "kernel": ("k_force_n3_f32c + k_n3_reduce (Newton-3: each unordered pair evaluated once)"
+                "kernel": ("k_strip_f32c + k_strip_reduce (Newton-3: each unordered pair evaluated once)"
                            if newton3 else f"k_force_f32c<{cfg[0]},{cfg[1]}> split {cfg[2]}"),
                 "fma_ops_per_ordered_pair": ops,
                 "traffic_note": "dram bytes per launch of the pair kernel from "

@@ -328,8 +328,8 @@ int nbr_get_force_tiling(nbr_ctx* ctx, int precision, double eps2, int* tile, in
 /* The configuration a force evaluation of the uploaded system would use
  * (forced, autotuned or default): ni = 4 or 8 receivers per thread of the
  * large kernels, ni = 1 the small-N kernel (warps = lane groups per warp),
- * ni = 3 the Newton-3 kernel (each unordered pair once; the default of both
- * precisions from 16384 to 2^20 particles); split = j splits (unused by the
+ * ni = 3 the Newton-3 kernels (each unordered pair once; the default of both
+ * precisions from 4097 to 2^23 particles); split = j splits (unused by the
  * Newton-3 kernel). */
 int nbr_get_force_config(nbr_ctx* ctx, int precision, double eps2, int* ni, int* warps, int* split);
 /* Times the supported configurations for the uploaded system and stores the

@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32)
       const double* sy = sx + kTile;
       const double* sz = sy + kTile;
       const double* sm = sz + kTile;
-#pragma unroll 2
+#pragma unroll 4  // N = 16384, F = 8: 926 GPairs/s unrolled by 2, 961 by 4
       for (int j = phase; j < kTile; j += F) {
         const double xj = sx[j], yj = sy[j], zj = sz[j], mj = sm[j];
 #pragma unroll
