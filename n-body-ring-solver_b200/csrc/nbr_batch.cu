@@ -1417,6 +1417,21 @@ int nbr_batch_upload(nbr_ctx* c, size_t nsys, const size_t* offsets, const doubl
   return NBR_OK;
 }
 
+namespace {
+// The rows of one padded device array into dst, by way of h.
+cudaError_t fetch_padded(nbr_ctx* c, std::vector<double>& h, double* dst, const double* d) {
+  const BatchState& b = c->bat;
+  h.resize(b.s.n_pad);
+  cudaError_t e =
+      cudaMemcpyAsync(h.data(), d, b.s.n_pad * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  if (e != cudaSuccess) return e;
+  for (size_t s = 0; s < b.nsys; ++s)
+    std::memcpy(dst + b.off[s], &h[b.poff[s]], (b.off[s + 1] - b.off[s]) * sizeof(double));
+  return cudaSuccess;
+}
+}  // namespace
+
 int nbr_batch_download(nbr_ctx* c, double* x, double* y, double* z, double* vx, double* vy,
                        double* vz) {
   TraceRange trace_range("nbr_batch_download");
@@ -1425,15 +1440,24 @@ int nbr_batch_download(nbr_ctx* c, double* x, double* y, double* z, double* vx, 
   if (b.nsys == 0) return fail(c, NBR_ERR_NO_SYSTEM, "no batch uploaded");
   cudaSetDevice(c->device);
   cudaError_t e = cudaSuccess;
-  if (!b.d_flat) e = dalloc((void**)&b.d_flat, 6 * b.n_real * sizeof(double));
-  if (e != cudaSuccess) return cuda_fail(c, e, "batch download buffer");
   const int a = b.s.cur;
+  double* out[6] = {x, y, z, vx, vy, vz};
+  if (!b.d_flat && dalloc((void**)&b.d_flat, 6 * b.n_real * sizeof(double)) != cudaSuccess) {
+    // no room on the device: the padding is taken out on the host
+    cudaGetLastError();
+    b.d_flat = nullptr;
+    const double* src[6] = {b.s.pos[a][0], b.s.pos[a][1], b.s.pos[a][2],
+                            b.s.vel[0], b.s.vel[1], b.s.vel[2]};
+    std::vector<double> h;
+    for (int f = 0; f < 6; ++f)
+      if (out[f] && e == cudaSuccess) e = fetch_padded(c, h, out[f], src[f]);
+    return e == cudaSuccess ? NBR_OK : cuda_fail(c, e, "batch download");
+  }
   const BatchRows rows{{b.s.pos[a][0], b.s.pos[a][1], b.s.pos[a][2], b.s.vel[0], b.s.vel[1], b.s.vel[2]}};
   const long long ntiles = b.poff[b.nsys] / kTile;
   k_batch_flatten<<<(unsigned)((ntiles + 3) / 4), 128, 0, c->stream>>>(
       rows, b.d_flat, (long long)b.n_real, b.d_poff, b.d_off, (int)b.nsys, ntiles);
   e = cudaGetLastError();
-  double* out[6] = {x, y, z, vx, vy, vz};
   for (int f = 0; f < 6; ++f)
     if (out[f] && e == cudaSuccess)
       e = cudaMemcpyAsync(out[f], b.d_flat + f * b.n_real, b.n_real * sizeof(double),

@@ -17,6 +17,7 @@
 #include <fstream>
 #include <map>
 #include <mutex>
+#include <new>
 #include <sstream>
 #include <string>
 #include <vector>
@@ -427,7 +428,7 @@ StripLaunches strip_launches(nbr_ctx* c, int precision) {
   StripLaunches L;
   const long long n = (long long)c->sys.n;
   L.ni = strip_choose(precision, n, c->sms);
-  L.cut = strip_bands(precision, n, c->sms, L.ni, forced_bands());
+  L.cut = strip_bands(precision, n, c->sms, L.ni, forced_bands(), c->strip_single);
   for (size_t v = 0; v + 1 < L.cut.size(); ++v)
     L.doubles = std::max(
         L.doubles, strip_plan(precision, n, L.cut[v], L.cut[v + 1], c->sms, L.ni).doubles);
@@ -448,7 +449,19 @@ bool uses_strips(int precision, const ForceConfig& cfg, long long n) {
 // Prepares scratch for a force launch of `cfg` over n_i receivers.
 int prepare_split(nbr_ctx* c, int precision, const ForceConfig& cfg, long long n_pad_i) {
   if (uses_strips(precision, cfg, (long long)c->sys.n)) {  // (the context's whole system only)
-    const cudaError_t e = c->scr.need_part((size_t)strip_launches(c, precision).doubles);
+    long long doubles = strip_launches(c, precision).doubles;
+    cudaError_t e = c->scr.need_part((size_t)doubles);
+    if (e == cudaErrorMemoryAllocation && doubles > kN3SliceMaxDoubles &&
+        c->strip_single > kN3SliceMaxDoubles) {
+      // No room for one launch's scratch (up to 9 GiB; the CTA grid, which
+      // took 0.6 of it, may have found room): several launches of 2 GiB.  A
+      // graph captured with the larger scratch must not run on the smaller.
+      cudaGetLastError();
+      for (RunGraph& g : c->run_graph) g.release();
+      c->strip_single = kN3SliceMaxDoubles;
+      doubles = strip_launches(c, precision).doubles;
+      e = c->scr.need_part((size_t)doubles);
+    }
     return e == cudaSuccess ? NBR_OK : cuda_fail(c, e, "Newton-3 scratch");
   }
   if (cfg.ni == 3) {  // Newton-3 (the context's whole system only): its own partial sums
@@ -493,10 +506,27 @@ int check_device_error(nbr_ctx* c) {
   return device_error_status(c, h);
 }
 
+bool stage_host(nbr_ctx* c, size_t doubles) {
+  if (c->h_stage.size() >= doubles) return true;
+  try {
+    c->h_stage.resize(doubles);
+  } catch (const std::bad_alloc&) {
+    return false;
+  }
+  return true;
+}
+
+bool stage_ready(nbr_ctx* c, size_t doubles) {
+  if (!stage_host(c, doubles)) return false;
+  if (c->scr.need_red(doubles) == cudaSuccess) return true;
+  cudaGetLastError();
+  return false;
+}
+
 cudaError_t stage_fetch(nbr_ctx* c, const StageArrays& a, double* dst, int words[2]) {
   size_t total = 0;
   for (int k = 0; k < a.count; ++k) total += (size_t)a.n[k];
-  c->h_stage.resize(std::max(c->h_stage.size(), total + 1));
+  if (!stage_host(c, total + 1)) return cudaErrorMemoryAllocation;
   cudaError_t e = launch_stage_out(a, dst, c->d_err, c->stream);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(c->h_stage.data(), dst, (total + 1) * sizeof(double),
@@ -522,9 +552,9 @@ cudaError_t stage_download(nbr_ctx* c, int count, const double* const* src, doub
   int words[2] = {0, 0};
   if (e == cudaSuccess) e = stage_fetch(c, a, c->scr.red, words);
   if (e != cudaSuccess) return e;
-  *err = words[0];
+  if (err) *err = words[0];
   if (flags) *flags = words[1];
-  if (*err == kErrNone && !(flags && *flags))
+  if (!(err && *err != kErrNone) && !(flags && *flags))
     for (int k = 0; k < arrays; ++k)
       std::memcpy(to[k], c->h_stage.data() + (size_t)k * n, n * sizeof(double));
   return cudaSuccess;
@@ -903,6 +933,7 @@ int nbr_system_upload(nbr_ctx* c, size_t n, const double* x, const double* y, co
   if (e != cudaSuccess) return cuda_fail(c, e, "system allocation");
   s.cur = 0;
   s.rec_ok[0] = s.rec_ok[1] = false;
+  c->strip_single = kN3SingleMaxDoubles;
   c->acc_ok = false;
   const size_t B = n * sizeof(double);
   auto H = [&](double* d, const double* h) {
@@ -948,14 +979,12 @@ int nbr_system_download(nbr_ctx* c, double* x, double* y, double* z, double* vx,
   cudaSetDevice(c->device);
   const size_t B = s.n * sizeof(double);
   cudaError_t e = cudaSuccess;
-  if (stage_fits(6 * s.n)) {
+  if (stage_fits(6 * s.n) && stage_ready(c, 6 * s.n + 2)) {
     const double* src[6] = {s.pos[s.cur][0], s.pos[s.cur][1], s.pos[s.cur][2],
                             s.vel[0], s.vel[1], s.vel[2]};
     double* out[6] = {x, y, z, vx, vy, vz};
-    int err = 0;
-    e = stage_download(c, 6, src, out, s.n, &err);
-    if (e != cudaSuccess) return cuda_fail(c, e, "download");
-    return device_error_status(c, err);
+    e = stage_download(c, 6, src, out, s.n, nullptr);
+    return e == cudaSuccess ? NBR_OK : cuda_fail(c, e, "download");
   }
   auto D = [&](double* h, const double* d) {
     if (h && e == cudaSuccess) e = cudaMemcpyAsync(h, d, B, cudaMemcpyDeviceToHost, c->stream);
@@ -979,7 +1008,7 @@ int nbr_forces(nbr_ctx* c, int precision, double G, double eps2, int want_force,
   cudaSetDevice(c->device);
   int rc = eval_system(c, precision, G, eps2, 0, 0.0, 0.0, want_force, nullptr);
   if (rc) return rc;
-  const bool staged = stage_fits(3 * s.n);
+  const bool staged = stage_fits(3 * s.n) && stage_ready(c, 3 * s.n + 2);
   if (staged) {
     const double* src[3] = {s.acc[0], s.acc[1], s.acc[2]};
     double* out[3] = {ax, ay, az};
@@ -1204,7 +1233,12 @@ int nbr_accel_ij(nbr_ctx* c, int precision, size_t n_i, const double* xi, const 
     return fail(c, NBR_ERR_INVALID_ARG, "eps2 must be finite and >= 0, G finite");
   if (n_i > (size_t)1 << 31 || n_j > (size_t)1 << 31) return fail(c, NBR_ERR_INVALID_ARG, "size above 2^31");
   // small sets: one transfer each way, the check on the device
-  const bool staged = n_j > 0 && stage_fits((mi ? 4 : 3) * n_i + 4 * n_j);
+  const size_t total = (mi ? 4 : 3) * n_i + 4 * n_j;
+  bool staged = n_j > 0 && stage_fits(total);
+  if (staged) {
+    cudaSetDevice(c->device);
+    staged = stage_ready(c, total + 2);  // (3 n_i + 2 come back)
+  }
   if (!staged &&
       (!finite_array(xi, n_i) || !finite_array(yi, n_i) || !finite_array(zi, n_i) ||
        (mi && !finite_array(mi, n_i)) || !finite_array(xj, n_j) || !finite_array(yj, n_j) ||
@@ -1230,10 +1264,6 @@ int nbr_accel_ij(nbr_ctx* c, int precision, size_t n_i, const double* xi, const 
   if (staged) {
     StageArrays sa{};
     size_t off = 0;
-    const size_t total = (mi ? 4 : 3) * n_i + 4 * n_j;
-    c->h_stage.resize(std::max(c->h_stage.size(), total));
-    e = c->scr.need_red(total);
-    if (e != cudaSuccess) return cuda_fail(c, e, "ij staging");
     auto put = [&](double* d, const double* h, size_t n, long long np) {
       if (!h) return;
       std::memcpy(c->h_stage.data() + off, h, n * sizeof(double));

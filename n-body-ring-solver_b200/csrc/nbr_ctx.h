@@ -135,11 +135,15 @@ int device_error_status(nbr_ctx* c, int h);
 // the host.
 constexpr size_t kStageBytes = 1 << 20;
 inline bool stage_fits(size_t doubles) { return doubles * sizeof(double) <= kStageBytes; }
+// Whether both sides hold `doubles` (allocated here where they do not): a call
+// whose staging finds no memory makes its transfers one by one.
+bool stage_ready(nbr_ctx* c, size_t doubles);
 // The arrays of a, packed at dst (device scratch), into c->h_stage, and the
 // device error block's first two words into words; waits for the stream.
 cudaError_t stage_fetch(nbr_ctx* c, const StageArrays& a, double* dst, int words[2]);
 // count arrays of n doubles each into out[k] (null: left out), unless *err (the
-// device error word) or *flags (the input flags) is set.
+// device error word) or *flags (the input flags) is set.  err null: whatever the
+// error word, which stays for the next call that checks it.
 cudaError_t stage_download(nbr_ctx* c, int count, const double* const* src, double* const* out,
                            size_t n, int* err, int* flags = nullptr);
 // Bounded-wait limit and tile-skip test hook from the environment.
@@ -206,6 +210,9 @@ struct nbr_ctx {
   // between two.
   nbr::RunGraph run_graph[nbr::kRunGraphs];
   std::vector<double> h_stage;
+  // Most scratch of an evaluation in strips that runs as one launch, lowered
+  // when that much could not be allocated, until the next upload.
+  long long strip_single = nbr::kN3SingleMaxDoubles;
   // The last persistent launch configuration whose attributes were set, and its
   // resident CTAs per SM.
   const void* persist_fn = nullptr;

@@ -253,8 +253,10 @@ struct StripPlan {
 StripPlan strip_plan(int precision, long long n, int r0, int r1, int sms, int ni);
 // Receivers per lane for a whole system.
 int strip_choose(int precision, long long n, int sms);
-// The row blocks at which an evaluation's launches begin and, last, their count.
-std::vector<int> strip_bands(int precision, long long n, int sms, int ni, int bands);
+// The row blocks at which an evaluation's launches begin and, last, their count:
+// one launch up to single_max doubles of scratch, or `bands` launches if > 0.
+std::vector<int> strip_bands(int precision, long long n, int sms, int ni, int bands,
+                             long long single_max);
 // The strips of plan p over the FP64 particles of js (the receivers ip are the
 // same particles), then the reduction: mode 0 runs the epilogue ep (which
 // writes no FP32C records), 1 stores the accelerations over G of all particles

@@ -617,9 +617,10 @@ int strip_choose(int precision, long long n, int sms) {
 }
 
 // Row blocks of each launch of an evaluation: all of them where the partial
-// sums fit kN3SingleMaxDoubles, else launches of at most kN3SliceMaxDoubles
+// sums fit single_max (kN3SingleMaxDoubles), else launches of at most kN3SliceMaxDoubles
 // (bands > 0: that many launches, for the tests).
-std::vector<int> strip_bands(int precision, long long n, int sms, int ni, int bands) {
+std::vector<int> strip_bands(int precision, long long n, int sms, int ni, int bands,
+                             long long single_max) {
   const int rows = (int)((n + 32 * ni - 1) / (32 * ni));
   std::vector<int> cut{0};
   if (bands > 0) {
@@ -636,7 +637,7 @@ std::vector<int> strip_bands(int precision, long long n, int sms, int ni, int ba
     return ((long long)sms * kStripWarps + r1 - r0) * 96 * ni +
            96 * (std::max(0LL, units) + ni) / (precision == kFP32C ? 2 : 1);
   };
-  if (doubles(0, rows) <= kN3SingleMaxDoubles) {
+  if (doubles(0, rows) <= single_max) {
     cut.push_back(rows);
     return cut;
   }

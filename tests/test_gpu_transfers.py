@@ -83,3 +83,62 @@ def test_batch_download_is_the_upload(ctx, nbr):
     got = ctx.batch_download()
     for k in ("x", "y", "z", "vx", "vy", "vz"):
         np.testing.assert_array_equal(got[k], st[k])
+
+
+# Where there is no room for what a transfer or a launch would take at its
+# fastest, the call does without it: the same results.
+def failing_allocation(monkeypatch, call, k="1"):
+    monkeypatch.setenv("NBR_TEST_FAIL_ALLOC", k)
+    try:
+        return call()
+    finally:
+        monkeypatch.delenv("NBR_TEST_FAIL_ALLOC")
+
+
+def test_transfers_without_staging(nbr, monkeypatch):
+    s = nbr.plummer(1500, 5)
+    with nbr.Context(0) as c:
+        c.upload(s)
+        got = failing_allocation(monkeypatch, c.download)
+        for k in ("x", "y", "z", "vx", "vy", "vz"):
+            np.testing.assert_array_equal(got[k], s[k])
+    args = [s[k] for k in ("x", "y", "z", "x", "y", "z", "m")]
+    with nbr.Context(0) as c:
+        a = failing_allocation(monkeypatch, lambda: c.accel_ij(*args, eps2=1e-4))
+        np.testing.assert_array_equal(a, c.accel_ij(*args, eps2=1e-4))
+    off = np.array([0, 300, 1500])
+    with nbr.Context(0) as c:
+        c.batch_upload(off, s)
+        got = failing_allocation(monkeypatch, c.batch_download)
+        for k in ("x", "y", "z", "vx", "vy", "vz"):
+            np.testing.assert_array_equal(got[k], s[k])
+        np.testing.assert_array_equal(c.batch_download()["x"], s["x"])
+
+
+def test_strips_in_less_scratch(nbr, monkeypatch):
+    """450000 particles take 2.4 GB of reactions in one launch."""
+    with nbr.Context(0) as c:
+        c.upload(nbr.plummer(450000, 5))
+        few = failing_allocation(monkeypatch, lambda: c.forces(FP32C, eps2=1e-4))
+        again = c.forces(FP32C, eps2=1e-4)
+        np.testing.assert_array_equal(few, again)
+        c.upload(nbr.plummer(450000, 5))
+        e = rel_err(few, c.forces(FP32C, eps2=1e-4))
+        assert np.median(e) <= 1e-6 and e.max() <= 1e-4
+
+
+def test_download_leaves_a_pending_error(nbr, monkeypatch):
+    """A download after an evaluation that timed out returns the state; the
+    status is the next evaluation's, as for arrays too large to be packed."""
+    s = nbr.plummer(5000, 5)
+    with nbr.Context(0) as c:
+        c.upload(s)
+        c.set_force_config(FP64, 4, 4)
+        monkeypatch.setenv("NBR_WAIT_LIMIT_MS", "50")
+        monkeypatch.setenv("NBR_TEST_SKIP_TILE", "1")
+        c.forces_device(FP64, eps2=1e-4)
+        monkeypatch.delenv("NBR_TEST_SKIP_TILE")
+        np.testing.assert_array_equal(c.download()["x"], s["x"])
+        with pytest.raises(nbr.NbrError):
+            c.synchronize()
+        assert np.isfinite(c.forces(FP64, eps2=1e-4)).all()
