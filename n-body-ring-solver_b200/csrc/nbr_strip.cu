@@ -45,7 +45,7 @@ __host__ __device__ inline int strip_prefix(const StripPlan& p, int r) {
   return (int)((long long)(r - p.r0) * p.batches -
                (long long)p.tb * (((long long)r * (r - 1) - (long long)p.r0 * (p.r0 - 1)) / 2));
 }
-// First element of row block r's reactions.
+// First element of row block r's reactions: [batch after its own][3][32].
 __host__ __device__ inline long long strip_rea_off(const StripPlan& p, int r) {
   return 96 * ((long long)(r - p.r0) * p.batches -
                (long long)p.tb * (((long long)r * (r + 1) - (long long)p.r0 * (p.r0 + 1)) / 2));
@@ -142,13 +142,13 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
     u += b1 - b0;
     const long long ibase = (long long)r * (32 * NI) + lane;
     const int b_rea = (r + 1) * TB;  // first batch whose reactions are kept
-    const long long len = 32LL * (sp.batches - b_rea);
+    const long long len = 96LL * (sp.batches - b_rea);  // reactions of this row block
     if (!NBR_IN((long long)(r + 1) * (32 * NI) - 1, ip.len, err) ||
         !NBR_IN(32LL * (((b1 - 1) | 3) + 1) - 1, js.len, err) ||
         !NBR_IN((long long)(g + r - sp.r0 + 1) * (96 * NI) - 1, sp.act_doubles, err) ||
-        (len > 0 && !NBR_IN(strip_rea_off(sp, r) + 3 * len - 1, sp.reactions, err)))
+        (len > 0 && !NBR_IN(strip_rea_off(sp, r) + len - 1, sp.reactions, err)))
       return;
-    float* out = rea + strip_rea_off(sp, r) + lane - 32LL * b_rea;
+    float* out = rea + strip_rea_off(sp, r) + lane - 96LL * b_rea;
     u64 MI[IP];
 #pragma unroll
     for (int p = 0; p < IP; ++p)
@@ -246,11 +246,11 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
           sm = __shfl_sync(0xffffffffu, sm, from);
         }
         if (b >= b_rea) {
-          float* o = out + 32LL * b;
+          float* o = out + 96LL * b;
           float l, h;
           unpack2(RX, l, h); o[0] = -(l + h);
-          unpack2(RY, l, h); o[len] = -(l + h);
-          unpack2(RZ, l, h); o[2 * len] = -(l + h);
+          unpack2(RY, l, h); o[32] = -(l + h);
+          unpack2(RZ, l, h); o[64] = -(l + h);
         }
       }
 #pragma unroll
@@ -308,13 +308,13 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
     u += b1 - b0;
     const long long ibase = (long long)r * (32 * NI) + lane;
     const int b_rea = (r + 1) * TB;
-    const long long len = 32LL * (sp.batches - b_rea);
+    const long long len = 96LL * (sp.batches - b_rea);  // reactions of this row block
     if (!NBR_IN((long long)(r + 1) * (32 * NI) - 1, ip.len, err) ||
         !NBR_IN(32LL * (((b1 - 1) | 3) + 1) - 1, js.len, err) ||
         !NBR_IN((long long)(g + r - sp.r0 + 1) * (96 * NI) - 1, sp.act_doubles, err) ||
-        (len > 0 && !NBR_IN(strip_rea_off(sp, r) + 3 * len - 1, sp.reactions, err)))
+        (len > 0 && !NBR_IN(strip_rea_off(sp, r) + len - 1, sp.reactions, err)))
       return;
-    double* out = rea + strip_rea_off(sp, r) + lane - 32LL * b_rea;
+    double* out = rea + strip_rea_off(sp, r) + lane - 96LL * b_rea;
     double xi[NI], yi[NI], zi[NI], mi[NI], ax[NI], ay[NI], az[NI];
 #pragma unroll
     for (int k = 0; k < NI; ++k) {
@@ -375,10 +375,10 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
         xs = xn; ys = yn; zs = zn; ms = mn;
       }
       if (b >= b_rea) {
-        double* o = out + 32LL * b;
+        double* o = out + 96LL * b;
         o[0] = -RX;
-        o[len] = -RY;
-        o[2 * len] = -RZ;
+        o[32] = -RY;
+        o[64] = -RZ;
       }
       if ((b & 3) == 3 || b + 1 == b1) {
 #pragma unroll
@@ -497,10 +497,21 @@ __global__ void __launch_bounds__(kStripWarps * 32, NI == 4 ? 2 : 1)
 // system) and then over the warps in order: a fixed order.  By mode: 0 runs the
 // epilogue of the large kernels, 1 stores the sums into dst[d * ld + i], 2
 // adds them to it (a launch over some of the row blocks).
+//
+// What bounds it: on a small system the chain of loads, on a large one the bytes
+// of the reactions in flight (0.8 GB at N = 262144 FP32C).  So up to two CTAs per
+// SM in all each warp has eight row blocks' loads in flight; above that four, in
+// 40 registers, so that three CTAs share an SM.  The reactions lie by (row
+// block, batch), 384 or 768 bytes together, which strip and reduction move as
+// one piece.  us per evaluation: before (one array per component, four row
+// blocks, two CTAs) / two CTAs and eight / three CTAs and four: FP32C N = 4224
+// 15.6 / 15.5 / 16.4, 12001 61.1 / 60.1 / 58.1, 65536 1385 / 1375 / 1366, 262144
+// 21743 / 21576 / 21510; FP64 4224 21.4 / 21.1 / 22.0, 12001 112.4 / 112.4 / 110.1,
+// 16000 180.6 / 181.9 / 181.2, 196608 25214 / 25072 / 25042.
 constexpr int kRedWarps = 16;
 
-template <int PREC>
-__global__ void __launch_bounds__(32 * kRedWarps)
+template <int PREC, int PER_SM>
+__global__ void __launch_bounds__(32 * kRedWarps, PER_SM)
     k_strip_reduce(const IParticles ip, const Epilogue ep, const StripPlan sp, const double* act,
                    const void* rea_v, const double scale, const int mode, double* dst,
                    const long long ld) {
@@ -529,11 +540,11 @@ __global__ void __launch_bounds__(32 * kRedWarps)
   // the reactions from the row blocks before its own
   const T* rea = reinterpret_cast<const T*>(rea_v);
   const int r_end = min(rb, sp.r1);
-#pragma unroll 4
+  constexpr int kRows = PER_SM == 2 ? 8 : 4;
+#pragma unroll kRows
   for (int r = sp.r0 + ph; r < r_end; r += kRedWarps) {
-    const long long first = 32LL * sp.tb * (r + 1), len = 32LL * sp.batches - first;
-    const T* a = rea + strip_rea_off(sp, r) + (i - first);
-    sx += (double)a[0]; sy += (double)a[len]; sz += (double)a[2 * len];
+    const T* a = rea + strip_rea_off(sp, r) + 96LL * (b - sp.tb * (r + 1)) + lane;
+    sx += (double)a[0]; sy += (double)a[32]; sz += (double)a[64];
   }
   part[ph][0][lane] = sx; part[ph][1][lane] = sy; part[ph][2][lane] = sz;
   __syncthreads();
@@ -731,11 +742,12 @@ cudaError_t launch_strips(int precision, const StripPlan& p, double eps2, const 
   cfg.blockDim = dim3(32 * kRedWarps);
   cfg.dynamicSmemBytes = 0;
   const void* sums = rea;
+  const bool small = p.batches <= 2 * sms;
   if (precision == kFP32C)
-    return cudaLaunchKernelEx(&cfg, k_strip_reduce<kFP32C>, ip, ep, p, (const double*)act, sums,
-                              1.0 / ((double)kC53 - 1.0), mode, dst, ld);
-  return cudaLaunchKernelEx(&cfg, k_strip_reduce<kFP64>, ip, ep, p, (const double*)act, sums,
-                            kInvCubeScale, mode, dst, ld);
+    return cudaLaunchKernelEx(&cfg, small ? k_strip_reduce<kFP32C, 2> : k_strip_reduce<kFP32C, 3>, ip,
+                              ep, p, (const double*)act, sums, 1.0 / ((double)kC53 - 1.0), mode, dst, ld);
+  return cudaLaunchKernelEx(&cfg, small ? k_strip_reduce<kFP64, 2> : k_strip_reduce<kFP64, 3>, ip, ep,
+                            p, (const double*)act, sums, kInvCubeScale, mode, dst, ld);
 }
 
 }  // namespace nbr

@@ -60,6 +60,17 @@ def test_default_strips(ctx, nbr, oracle, prec, n):
         del os.environ["NBR_TEST_N3_SLICES"]
 
 
+# two CTAs of the reduction per SM in all, and one batch more: 148 SMs, 296 batches
+@pytest.mark.parametrize("prec", [FP64, FP32C])
+@pytest.mark.parametrize("n", [9471, 9472, 9473, 9505])
+def test_reduction_where_its_form_changes(ctx, nbr, oracle, prec, n):
+    s = nbr.plummer(n, n)
+    ctx.upload(s)
+    idx = np.unique(np.concatenate([np.arange(0, n, 97), np.arange(n - 40, n)]))
+    ref = oracle.accel_subset(s["x"], s["y"], s["z"], s["m"], idx, eps2=1e-6)
+    check(ctx.forces(prec, eps2=1e-6)[:, idx], ref, prec)
+
+
 @pytest.mark.parametrize("m0", [0.0, -1.3, 0.7, 1.99999999, 1e-30, 5e-324])
 def test_strips_any_mass_of_particle_0(ctx, nbr, oracle, m0):
     """FP32C strips take particle 0's mass mantissa as their unit of mass."""
