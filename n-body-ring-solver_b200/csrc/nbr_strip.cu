@@ -101,23 +101,10 @@ __device__ __forceinline__ void launch_dependents() {
 // next one (2805 -> 2912); sources by shuffle rather than from shared memory
 // (3133 against 3166 at NI = 16).
 //
-// Masses are divided by the mantissa of particle 0's before they are rounded to
-// FP32, and the sums multiplied by it: equal masses, and whole ratios of them,
-// then carry no rounding at all, and no mass changes by more than a factor of
-// two.  (Rounded masses act with up to 6e-8 too much or too little, the same in
-// every step: 2.1e-9 of energy drift over 500 steps of 131072 bodies of
-// masses 1 and 1000 with FP32 masses, 6.3e-10 with scaled ones, 3.2e-10 in FP64.)
-//
 // Coordinates are relative to the tile's FP64 origin, the mean of its 128
 // particles, in FP32; per tile of 128 sources the FP32 action sums are added
 // to FP64 sums.
 constexpr float kC53 = 1.66666663f;
-// The mantissa of m, in [1, 2) (1 for zero and subnormal masses).
-__device__ __forceinline__ double mass_mantissa(double m) {
-  const int hi = __double2hiint(m);
-  return hi < 0x00100000 ? 1.0
-                         : __hiloint2double((hi & 0x000fffff) | 0x3ff00000, __double2loint(m));
-}
 
 template <int NI, bool EXCL>
 __global__ void __launch_bounds__(kStripWarps * 32, 1)
@@ -135,7 +122,6 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
   const int from = (lane + 31) & 31;
   const u64 EPS2 = pack2(eps2f, eps2f), C53 = pack2(kC53, kC53);
   double* acc = strip_acc + warp * (96 * NI) + lane;
-  const double unit = 1.0 / mass_mantissa(js.m[0]);  // the kernel's unit of mass
   for (int r = strip_row(sp, u); u < u_end; ++r) {
     const int b0 = r * TB + (u - strip_prefix(sp, r));
     const int b1 = min(sp.batches, b0 + (u_end - u));
@@ -152,7 +138,7 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
     u64 MI[IP];
 #pragma unroll
     for (int p = 0; p < IP; ++p)
-      MI[p] = pack2((float)(unit * ip.m[ibase + 64 * p]), (float)(unit * ip.m[ibase + 64 * p + 32]));
+      MI[p] = pack2((float)ip.m[ibase + 64 * p], (float)ip.m[ibase + 64 * p + 32]);
 #pragma unroll
     for (int k = 0; k < 3 * NI; ++k) acc[32 * k] = 0.0;
 #pragma unroll 1
@@ -191,7 +177,7 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
       for (; b < b_tile; ++b) {
         const long long j = 32LL * b + lane;
         float sx = __double2float_rn(js.x[j] - ox), sy = __double2float_rn(js.y[j] - oy),
-              sz = __double2float_rn(js.z[j] - oz), sm = (float)(unit * js.m[j]);
+              sz = __double2float_rn(js.z[j] - oz), sm = (float)js.m[j];
         u64 RX = 0ull, RY = 0ull, RZ = 0ull;
 #pragma unroll(NI >= 12 ? 2 : 4)
         for (int step = 0; step < 32; ++step) {
@@ -551,8 +537,7 @@ __global__ void __launch_bounds__(32 * kRedWarps, PER_SM)
   if (ph != 0) return;
 #pragma unroll
   for (int k = 1; k < kRedWarps; ++k) { sx += part[k][0][lane]; sy += part[k][1][lane]; sz += part[k][2][lane]; }
-  const double f = PREC == kFP32C ? scale * mass_mantissa(ip.m[0]) : scale;
-  sx *= f; sy *= f; sz *= f;
+  sx *= scale; sy *= scale; sz *= scale;
   if (mode == 1) { dst[i] = sx; dst[ld + i] = sy; dst[2 * ld + i] = sz; return; }
   if (mode == 2) { dst[i] += sx; dst[ld + i] += sy; dst[2 * ld + i] += sz; return; }
   if (i >= ip.n) return;

@@ -71,22 +71,6 @@ def test_reduction_where_its_form_changes(ctx, nbr, oracle, prec, n):
     check(ctx.forces(prec, eps2=1e-6)[:, idx], ref, prec)
 
 
-@pytest.mark.parametrize("m0", [0.0, -1.3, 0.7, 1.99999999, 1e-30, 5e-324])
-def test_strips_any_mass_of_particle_0(ctx, nbr, oracle, m0):
-    """FP32C strips take particle 0's mass mantissa as their unit of mass."""
-    n = 4500
-    s = nbr.plummer(n, 8)
-    s["m"][:] *= np.random.default_rng(1).uniform(0.1, 30.0, n)
-    s["m"][0] = m0
-    if m0 < 0:  # no unit to take: refused by the upload
-        with pytest.raises(nbr.NbrError):
-            ctx.upload(s)
-        return
-    ctx.upload(s)
-    ref = oracle.accel(s["x"], s["y"], s["z"], s["m"], eps2=1e-4, extended=True)
-    check(ctx.forces(FP32C, eps2=1e-4), ref, FP32C)
-
-
 @pytest.mark.parametrize("prec,tol", [(FP64, 1e-11), (FP32C, 1e-6)])
 @pytest.mark.parametrize("scheme", ["kdk", "euler"])
 def test_strip_runs_between_other_kernels(ctx, nbr, oracle, prec, tol, scheme):
