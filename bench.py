@@ -342,8 +342,8 @@ def run_ours(a):
     k32 = time_kernel(nbr.FP32C, 5)
     a32 = ctx.forces_download()
     # The plain FP64 kernel (every ordered pair), the one the FP32C / FP64
-    # ratio is defined on, then the FP64 default for this size (the Newton-3
-    # FP64 kernel from 16384 to 2^20 particles).
+    # ratio is defined on, then the FP64 default for this size (a Newton-3
+    # kernel above 4096 particles).
     ctx.set_force_config(nbr.FP64, 4, 4, 0)
     cfg64 = ctx.get_force_config(nbr.FP64, eps2)
     k64 = time_kernel(nbr.FP64, 3)

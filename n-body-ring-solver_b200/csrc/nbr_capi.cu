@@ -323,10 +323,10 @@ ForceConfig choose_config(nbr_ctx* c, int precision, double eps2, long long n_i,
     // FP32C is FMA-pipe bound and gains from 4 receiver pairs per thread;
     // FP64 has twice the registers per receiver and prefers 4 per thread.
     ForceConfig dflt = precision == kFP32C ? ForceConfig{8, 2, 0} : ForceConfig{4, 4, 0};
-    // Small systems: the warp-splitting kernel.  Lane groups per warp from a
-    // B200 sweep (forces per call, N = 256 .. 262144): FP32C 8 up to 4096
-    // receivers, 2 up to 8192; FP64 8 up to 16384, 4 up to 32768; above
-    // that the large kernels win.
+    // Small systems, receiver ranges and separate sets: the warp-splitting
+    // kernel.  Lane groups per warp from a B200 sweep (forces per call, N = 256
+    // .. 262144): FP32C 8 up to 4096 receivers, 2 up to 8192; FP64 8 up to
+    // 16384, 4 up to 32768; above that the large kernels win.
     const int F = precision == kFP32C ? (n_i <= 4096 ? 8 : n_i <= 8192 ? 2 : 0)
                                       : (n_i <= 16384 ? 8 : n_i <= 32768 ? 4 : 0);
     // From there to 2^23 particles: Newton-3 (B200, us per KDK step, the best
@@ -345,7 +345,7 @@ ForceConfig choose_config(nbr_ctx* c, int precision, double eps2, long long n_i,
   return cfg;
 }
 
-// The large-kernel default for callers that cannot take the Newton-3 kernel
+// The large-kernel default for callers that cannot take the Newton-3 kernels
 // (a receiver range, separate receiver and source sets).
 ForceConfig choose_config_large(nbr_ctx* c, int precision, double eps2, long long n_i, int ntiles) {
   ForceConfig cfg = precision == kFP32C ? ForceConfig{8, 2, 0} : ForceConfig{4, 4, 0};

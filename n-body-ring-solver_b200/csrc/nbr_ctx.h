@@ -218,7 +218,7 @@ struct nbr_ctx {
   const void* persist_fn = nullptr;
   size_t persist_smem = 0;
   int persist_per_sm = 0;
-  // Launch order of the whole-system Newton-3 grid (longest CTA first) for
+  // Launch order of the whole-system Newton-3 CTA grid (longest CTA first) for
   // n3_order_nb blocks, then its inverse; written before any graph capture
   // (n3_order_prepare, the only writer), read by the pair and reduce kernels.
   int* n3_order = nullptr;

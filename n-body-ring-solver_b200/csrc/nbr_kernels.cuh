@@ -204,10 +204,11 @@ inline long long n3_slice_scratch_doubles(long long nb, int v, int V) {
 }
 // One Newton-3 force evaluation over all n_pad receivers of ip against the
 // same particles in js (FP32C: their records; FP64: their x, y, z, m arrays),
-// with the epilogue ep: the pair kernel, then the per-particle reduction.
+// with the epilogue ep: the pair kernel, then the per-particle reduction.  The
+// default for FP64 above kStripMaxN64 particles (smaller ones and FP32C: strips).
 // scratch holds n3_scratch_doubles(ceil(n / kN3Block)) doubles; order is the
 // grid's launch order (n3_launch_order, on the device).
-// FP32C: warps = kN3Warps (one warp per row block) or kN3W2Warps (two).
+// FP32C: warps = kN3W2Warps (two warps per row block).
 cudaError_t launch_force_n3(int precision, int warps, double eps2, const IParticles& ip,
                             const JStream& js, const Epilogue& ep, double* scratch,
                             long long scratch_len, const int* order, cudaStream_t stream);
