@@ -104,6 +104,12 @@ __device__ __forceinline__ void launch_dependents() {
 // Coordinates are relative to the tile's FP64 origin, the mean of its 128
 // particles, in FP32; per tile of 128 sources the FP32 action sums are added
 // to FP64 sums.
+//
+// The padding lanes of the last batch take the last particle's coordinates,
+// with their own mass, zero: the pair factor multiplies the masses last, and at
+// that place it is inf or NaN only if it is for a real pair too.  (Where the
+// arrays hold the padding, at the coordinate origin, it may lie 1e20 units from
+// a particle, or 1e-14.)
 constexpr float kC53 = 1.66666663f;
 
 template <int NI, bool EXCL>
@@ -149,7 +155,8 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
       {
         const long long t0 = (long long)(b & ~3) * 32 + lane;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {  // padding sits at the origin: it adds nothing
+        for (int k = 0; k < 4; ++k) {
+          if (t0 + 32 * k >= ip.n) break;
           ox += js.x[t0 + 32 * k]; oy += js.y[t0 + 32 * k]; oz += js.z[t0 + 32 * k];
         }
 #pragma unroll
@@ -175,9 +182,9 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
       }
 #pragma unroll 1
       for (; b < b_tile; ++b) {
-        const long long j = 32LL * b + lane;
-        float sx = __double2float_rn(js.x[j] - ox), sy = __double2float_rn(js.y[j] - oy),
-              sz = __double2float_rn(js.z[j] - oz), sm = (float)js.m[j];
+        const long long j = 32LL * b + lane, jx = min(j, ip.n - 1);
+        float sx = __double2float_rn(js.x[jx] - ox), sy = __double2float_rn(js.y[jx] - oy),
+              sz = __double2float_rn(js.z[jx] - oz), sm = (float)js.m[j];
         u64 RX = 0ull, RY = 0ull, RZ = 0ull;
 #pragma unroll(NI >= 12 ? 2 : 4)
         for (int step = 0; step < 32; ++step) {

@@ -60,6 +60,35 @@ def test_default_strips(ctx, nbr, oracle, prec, n):
         del os.environ["NBR_TEST_N3_SLICES"]
 
 
+def ragged_last_batch(nbr, n, case):
+    s = {k: v.copy() for k, v in nbr.plummer(n, n).items() if k in "xyzm"}
+    if case == "far":  # the coordinate origin, 3e19 away, is no place for a source
+        s = {k: 1e10 * v for k, v in s.items()}
+        s["x"] += 3e19
+        return s, 1e14
+    # a body 1e-14 from the coordinate origin, last; the mean of its tile (alone,
+    # or with bodies in opposite pairs) as near
+    first = n - 1 - (n - 1) % 128
+    pairs = np.arange(first, n - 1).reshape(2, -1)
+    for k in "xyz":
+        s[k][pairs[1]] = -s[k][pairs[0]]
+        s[k][n - 1] = 1e-14 if k == "x" else 0.0
+    return s, 0.0
+
+
+# Massless padding of the last batch pulls nothing, wherever the system lies.
+@pytest.mark.parametrize("prec", [FP64, FP32C])
+@pytest.mark.parametrize("n", [4097, 4129, 8193])
+@pytest.mark.parametrize("case", ["far", "near"])
+def test_padding_of_the_last_batch(ctx, nbr, oracle, prec, n, case):
+    s, eps2 = ragged_last_batch(nbr, n, case)
+    ctx.upload(s)
+    assert ctx.get_force_config(prec, eps2)[0] == 3
+    idx = np.unique(np.concatenate([np.arange(0, n, 61), np.arange(n - 40, n)]))
+    ref = oracle.accel_subset(s["x"], s["y"], s["z"], s["m"], idx, eps2=eps2)
+    check(ctx.forces(prec, eps2=eps2)[:, idx], ref, prec)
+
+
 # two CTAs of the reduction per SM in all, and one batch more: 148 SMs, 296 batches
 @pytest.mark.parametrize("prec", [FP64, FP32C])
 @pytest.mark.parametrize("n", [9471, 9472, 9473, 9505])
