@@ -141,6 +141,14 @@ __device__ __noinline__ double inv_dist_tiny(double r2) {
   return rsqrt(r2) * (1.0 / kInvDistScale);
 }
 
+// Sum of p[0], p[ld], .. p[(K - 1) ld], K a power of two, by halves: the chain
+// of roundings (and of latencies) is log2 K long instead of K.
+template <int K>
+__device__ __forceinline__ double sum_by_halves(const double* p, int ld) {
+  if constexpr (K == 1) return *p;
+  else return sum_by_halves<K / 2>(p, ld) + sum_by_halves<K / 2>(p + K / 2 * ld, ld);
+}
+
 // Knuth TwoSum of the packed pair (hi + p): hi <- rounded sum, lo += the
 // rounding error.  Six packed adds; exact error term for round-to-nearest.
 __device__ __forceinline__ void two_sum2(u64& hi, u64& lo, u64 p) {

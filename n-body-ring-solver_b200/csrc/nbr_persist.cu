@@ -12,7 +12,7 @@
 //    shared memory with L2 loads, its W warps (8 or 16) split the sources W
 //    ways and the F lane groups of each warp split them again
 //    (k_force_small's layout), and the partial sums are combined in a fixed
-//    order (lane_sums, then the warps in order): deterministic;
+//    order (lane_sums, then the warps by halves): deterministic;
 //  * the CTA applies the fused kick/drift to its receivers, one thread per
 //    receiver and axis, whose velocities (and, FP32C, positions) stay in shared
 //    memory for the run, writes their positions to the next buffer, and all
@@ -265,7 +265,8 @@ __global__ void __launch_bounds__(W * 32, 1) k_run_small_f64(const PersistArgs A
           az[k] = fma(s, dz, az[k]);
         }
       }
-      // lane groups of the warp, then the warps in order
+      // lane groups of the warp, then the warps by halves (median error of an
+      // acceleration at N = 2048, in order / by halves: 1.11e-16 / 0.80e-16)
       double v[3 * kPNI];
 #pragma unroll
       for (int k = 0; k < kPNI; ++k) { v[3 * k] = ax[k]; v[3 * k + 1] = ay[k]; v[3 * k + 2] = az[k]; }
@@ -278,9 +279,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_run_small_f64(const PersistArgs A
       // a -> acc, v += kick a, x' = x + drift v (Euler: drift with the old velocity)
       if (threadIdx.x < 3 * RPC) {
         const int t = threadIdx.x / 3, d = threadIdx.x - 3 * t, i = base + t;
-        double a = 0.0;
-#pragma unroll
-        for (int w = 0; w < kPWarps; ++w) a += red[(size_t)w * RPC * 3 + threadIdx.x];
+        const double a = sum_by_halves<kPWarps>(red + threadIdx.x, RPC * 3);
         if (t < A.cs && i < n) {
           const double gx = A.G * (kInvCubeScale * a);
           if (e + 1 == A.evals) (d == 0 ? A.ax : d == 1 ? A.ay : A.az)[i] = gx;
@@ -494,9 +493,7 @@ __global__ void __launch_bounds__(kPW32 * 32, 1) k_run_small_f32c(const PersistA
       __syncthreads();
       if (threadIdx.x < 3 * RPC) {  // one thread per receiver and axis
         const int t = threadIdx.x / 3, d = threadIdx.x - 3 * t, i = base + t;
-        double a = 0.0;
-#pragma unroll
-        for (int w = 0; w < W; ++w) a += red[(size_t)w * RPC * 3 + threadIdx.x];
+        const double a = sum_by_halves<W>(red + threadIdx.x, RPC * 3);
         if (t < A.cs && i < n) {
           const double gx = A.G * a;
           if (e + 1 == A.evals) (d == 0 ? A.ax : d == 1 ? A.ay : A.az)[i] = gx;

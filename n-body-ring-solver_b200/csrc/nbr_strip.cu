@@ -271,12 +271,14 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
 // (lane groups, tiles, splits).  A strip's sources in one chain and the 32 NI
 // terms of a reaction in another made the error of a force 1.3 to 2 times as
 // large below 10000 particles.  So every 128 sources the action sums go to a
-// second level in shared memory (no cost measured), and with FINE a step's
+// second level in shared memory (no cost measured), with FINE a step's
 // NI reaction terms are added before they join the travelling sum (three more
 // adds per step, 2 % of the time; taken below kStripFine64, above it the sums
-// are more exact than before without it).  rms error over eps = 0 .. 1e-2,
-// before / now: N = 4500 1.55e-16 / 1.66e-16, 9000 1.57e-16 / 1.62e-16, 15000
-// 2.1e-16 / 1.8e-16, 100000 4.1e-16 / 1.8e-16.
+// are more exact than before without it), and the reduction adds its warps' sums
+// by halves (in order their last roundings alone made half of the error).
+// Median error of a force, eps = 0 .. 1e-2, the kernel before / now: N = 4200 1.05e-16 /
+// 0.86e-16, 9000 1.16e-16 / 0.84e-16, 14000 1.03e-16 / 0.92e-16, 32768 2.0e-16 /
+// 0.88e-16.
 constexpr long long kStripFine64 = 12288;
 template <int NI, bool EXCL, bool FINE>
 __global__ void __launch_bounds__(kStripWarps * 32, 1)
@@ -487,9 +489,9 @@ __global__ void __launch_bounds__(kStripWarps * 32, NI == 4 ? 2 : 1)
 // Adds the partial sums of a batch's 32 particles, one per lane: its row block's
 // strips, then the reactions from the row blocks before it, spread over the
 // CTA's warps (a particle's chain of loads is what takes the time on a small
-// system) and then over the warps in order: a fixed order.  By mode: 0 runs the
-// epilogue of the large kernels, 1 stores the sums into dst[d * ld + i], 2
-// adds them to it (a launch over some of the row blocks).
+// system); the warps' sums are then added by halves, one warp per axis: a fixed
+// order.  By mode: 0 runs the epilogue of the large kernels, 1 stores the sums
+// into dst[d * ld + i], 2 adds them to it (a launch over some of the row blocks).
 //
 // What bounds it: on a small system the chain of loads, on a large one the bytes
 // of the reactions in flight (0.8 GB at N = 262144 FP32C).  So up to two CTAs per
@@ -541,27 +543,29 @@ __global__ void __launch_bounds__(32 * kRedWarps, PER_SM)
   }
   part[ph][0][lane] = sx; part[ph][1][lane] = sy; part[ph][2][lane] = sz;
   __syncthreads();
-  if (ph != 0) return;
-#pragma unroll
-  for (int k = 1; k < kRedWarps; ++k) { sx += part[k][0][lane]; sy += part[k][1][lane]; sz += part[k][2][lane]; }
-  sx *= scale; sy *= scale; sz *= scale;
-  if (mode == 1) { dst[i] = sx; dst[ld + i] = sy; dst[2 * ld + i] = sz; return; }
-  if (mode == 2) { dst[i] += sx; dst[ld + i] += sy; dst[2 * ld + i] += sz; return; }
+  if (ph > 2) return;  // warp d: the sum and the epilogue of axis d
+  const int d = ph;
+  const double* half = &part[0][d][lane];
+  double s = sum_by_halves<kRedWarps / 2>(half, 96);
+  __syncwarp();  // the other half's loads after these: 40 registers
+  s = scale * (s + sum_by_halves<kRedWarps / 2>(half + 48 * kRedWarps, 96));
+  if (mode == 1) { dst[d * ld + i] = s; return; }
+  if (mode == 2) { dst[d * ld + i] += s; return; }
   if (i >= ip.n) return;
-  if (ep.mode == 0) {
-    const double sc = ep.want_force ? ep.G * ip.m[i] : ep.G;
-    ep.ax[i] = sc * sx; ep.ay[i] = sc * sy; ep.az[i] = sc * sz;
-    return;
-  }
-  const double gx = ep.G * sx, gy = ep.G * sy, gz = ep.G * sz;
-  ep.ax[i] = gx; ep.ay[i] = gy; ep.az[i] = gz;
-  const double ux = ep.vx[i], uy = ep.vy[i], uz = ep.vz[i];
-  const double vx = ux + ep.kick * gx, vy = uy + ep.kick * gy, vz = uz + ep.kick * gz;
-  ep.vx[i] = vx; ep.vy[i] = vy; ep.vz[i] = vz;
-  const bool euler = ep.mode == 2;
-  ep.xn[i] = ip.x[i] + ep.drift * (euler ? ux : vx);
-  ep.yn[i] = ip.y[i] + ep.drift * (euler ? uy : vy);
-  ep.zn[i] = ip.z[i] + ep.drift * (euler ? uz : vz);
+  auto finish = [&](double* a_out, double* vel, const double* x, double* xn) {
+    if (ep.mode == 0) {
+      a_out[i] = (ep.want_force ? ep.G * ip.m[i] : ep.G) * s;
+      return;
+    }
+    const double g = ep.G * s;
+    a_out[i] = g;
+    const double u = vel[i], v = u + ep.kick * g;
+    vel[i] = v;
+    xn[i] = x[i] + ep.drift * (ep.mode == 2 ? u : v);
+  };
+  if (d == 0) finish(ep.ax, ep.vx, ip.x, ep.xn);
+  else if (d == 1) finish(ep.ay, ep.vy, ip.y, ep.yn);
+  else finish(ep.az, ep.vz, ip.z, ep.zn);
 }
 
 }  // namespace
