@@ -101,9 +101,24 @@ __device__ __forceinline__ void launch_dependents() {
 // next one (2805 -> 2912); sources by shuffle rather than from shared memory
 // (3133 against 3166 at NI = 16).
 //
-// Coordinates are relative to the tile's FP64 origin, the mean of its 128
-// particles, in FP32; per tile of 128 sources the FP32 action sums are added
-// to FP64 sums.
+// Coordinates are relative to the tile's FP64 origin in FP32; per tile of 128
+// sources the FP32 action sums are added to FP64 sums.  The origin is the mean of
+// the tile's 128 particles, one of the first 32 counted twice: which one goes
+// with the row block.
+//
+// Rounding: no more than in the kernels before (lane groups, tiles joined by
+// two_sum, reactions in FP64) takes two things.  With FINE a step's reaction
+// terms are added before they join the travelling sum, which is then a chain of
+// 32 additions instead of 16 NI.  And an origin of its own for each row block: a
+// source's coordinates are rounded anew for each, where with one origin all its
+// reactions carried the same displacement.  Median
+// error of a force (masses within a factor of three, eps 1e-3), before / one
+// chain and one origin / now: N = 6000 3.3e-8 / 4.2e-8 / 3.3e-8, 12001 3.7e-8 /
+// 4.7e-8 / 3.5e-8, 65536 3.6e-8 / 3.8e-8 / 3.1e-8, 262144 3.5e-8 / 3.5e-8 / 2.9e-8.
+// FINE costs 1 % at N = 12001 and 65536 (1364 -> 1384 us per evaluation) and 2.4 % at
+// 262144 (21.31 -> 21.83 ms); from kStripFine32 on the error is below the one
+// before without it (at 65536, one particle of a hundred 1000 times as heavy,
+// 4.8e-8 against 4.7e-8; at 131072 4.1e-8 against 4.2e-8).
 //
 // The padding lanes of the last batch take the last particle's coordinates,
 // with their own mass, zero: the pair factor multiplies the masses last, and at
@@ -112,7 +127,8 @@ __device__ __forceinline__ void launch_dependents() {
 // a particle, or 1e-14.)
 constexpr float kC53 = 1.66666663f;
 
-template <int NI, bool EXCL>
+constexpr long long kStripFine32 = 1LL << 17;
+template <int NI, bool EXCL, bool FINE>
 __global__ void __launch_bounds__(kStripWarps * 32, 1)
     k_strip_f32c(const IParticles ip, const JStream js, const StripPlan sp, const float eps2f,
                  double* act, float* rea, int* err) {
@@ -133,6 +149,7 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
     const int b1 = min(sp.batches, b0 + (u_end - u));
     u += b1 - b0;
     const long long ibase = (long long)r * (32 * NI) + lane;
+    const int twice = r & 31;        // the particle of a tile that counts twice for its origin
     const int b_rea = (r + 1) * TB;  // first batch whose reactions are kept
     const long long len = 96LL * (sp.batches - b_rea);  // reactions of this row block
     if (!NBR_IN((long long)(r + 1) * (32 * NI) - 1, ip.len, err) ||
@@ -149,15 +166,18 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
     for (int k = 0; k < 3 * NI; ++k) acc[32 * k] = 0.0;
 #pragma unroll 1
     for (int b = b0; b < b1;) {
-      // one tile of 4 batches: its origin is the mean of its real particles
+      // one tile of 4 batches and its origin; a ragged tile's particles are each
+      // taken several times
       const int b_tile = min(b1, (b & ~3) + 4);
       double ox = 0.0, oy = 0.0, oz = 0.0;
       {
-        const long long t0 = (long long)(b & ~3) * 32 + lane;
+        const long long t0 = (long long)(b & ~3) * 32;
+        const int left = (int)min(128LL, ip.n - t0);  // the tile's particles
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          if (t0 + 32 * k >= ip.n) break;
-          ox += js.x[t0 + 32 * k]; oy += js.y[t0 + 32 * k]; oz += js.z[t0 + 32 * k];
+          const int t = (lane + 32 * k) * left >> 7;
+          const double w = k == 0 && lane == twice ? 2.0 : 1.0;
+          ox = fma(w, js.x[t0 + t], ox); oy = fma(w, js.y[t0 + t], oy); oz = fma(w, js.z[t0 + t], oz);
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
@@ -165,11 +185,7 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
           oy += __shfl_xor_sync(0xffffffffu, oy, off);
           oz += __shfl_xor_sync(0xffffffffu, oz, off);
         }
-        const double cnt = (double)min(128LL, ip.n - (t0 - lane));
-        const double q = (lane == 0 ? ox : lane == 1 ? oy : oz) / cnt;
-        ox = __shfl_sync(0xffffffffu, q, 0);
-        oy = __shfl_sync(0xffffffffu, q, 1);
-        oz = __shfl_sync(0xffffffffu, q, 2);
+        ox *= 1.0 / 129.0; oy *= 1.0 / 129.0; oz *= 1.0 / 129.0;
       }
       u64 XI[IP], YI[IP], ZI[IP], AX[IP], AY[IP], AZ[IP];
 #pragma unroll
@@ -220,19 +236,20 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
           for (int p = 0; p < IP; ++p) y2[p] = mul2(y2[p], y[p]);
 #pragma unroll
           for (int p = 0; p < IP; ++p) c[p] = mul2(y2[p], c[p]);
+          u64 tx = RX, ty = RY, tz = RZ;  // FINE: the step's reaction alone
 #pragma unroll
           for (int p = 0; p < IP; ++p) {
             const u64 sj = mul2(c[p], SM), si = mul2(c[p], MI[p]);
-            RX = fma2(si, dx[p], RX);
-            RY = fma2(si, dy[p], RY);
-            RZ = fma2(si, dz[p], RZ);
+            tx = FINE && p == 0 ? mul2(si, dx[p]) : fma2(si, dx[p], tx);
+            ty = FINE && p == 0 ? mul2(si, dy[p]) : fma2(si, dy[p], ty);
+            tz = FINE && p == 0 ? mul2(si, dz[p]) : fma2(si, dz[p], tz);
             AZ[p] = fma2(sj, dz[p], AZ[p]);
             AY[p] = fma2(sj, dy[p], AY[p]);
             AX[p] = fma2(sj, dx[p], AX[p]);
           }
-          RX = __shfl_sync(0xffffffffu, RX, from);
-          RY = __shfl_sync(0xffffffffu, RY, from);
-          RZ = __shfl_sync(0xffffffffu, RZ, from);
+          RX = __shfl_sync(0xffffffffu, FINE ? add2(RX, tx) : tx, from);
+          RY = __shfl_sync(0xffffffffu, FINE ? add2(RY, ty) : ty, from);
+          RZ = __shfl_sync(0xffffffffu, FINE ? add2(RZ, tz) : tz, from);
           sx = __shfl_sync(0xffffffffu, sx, from);
           sy = __shfl_sync(0xffffffffu, sy, from);
           sz = __shfl_sync(0xffffffffu, sz, from);
@@ -658,23 +675,25 @@ std::vector<int> strip_bands(int precision, long long n, int sms, int ni, int ba
 
 namespace {
 
-template <int NI>
+template <int NI, bool FINE>
 const void* strip_f32c(bool excl) {
-  return excl ? (const void*)k_strip_f32c<NI, true> : (const void*)k_strip_f32c<NI, false>;
+  return excl ? (const void*)k_strip_f32c<NI, true, FINE> : (const void*)k_strip_f32c<NI, false, FINE>;
 }
 template <int NI, bool FINE>
 const void* strip_f64(bool excl) {
   return excl ? (const void*)k_strip_f64<NI, true, FINE> : (const void*)k_strip_f64<NI, false, FINE>;
 }
-const void* strip_fn(int precision, int ni, bool excl, bool fine) {
+template <bool FINE>
+const void* strip_fn(int precision, int ni, bool excl) {
   if (precision == kFP32C)
-    return ni == 8 ? strip_f32c<8>(excl) : ni == 10 ? strip_f32c<10>(excl)
-                                         : ni == 16 ? strip_f32c<16>(excl) : nullptr;
-  if (fine)
-    return ni == 6 ? strip_f64<6, true>(excl) : ni == 8 ? strip_f64<8, true>(excl)
-                                              : ni == 10 ? strip_f64<10, true>(excl) : nullptr;
-  return ni == 6 ? strip_f64<6, false>(excl) : ni == 8 ? strip_f64<8, false>(excl)
-                                             : ni == 10 ? strip_f64<10, false>(excl) : nullptr;
+    return ni == 8 ? strip_f32c<8, FINE>(excl) : ni == 10 ? strip_f32c<10, FINE>(excl)
+                                               : ni == 16 ? strip_f32c<16, FINE>(excl) : nullptr;
+  return ni == 6 ? strip_f64<6, FINE>(excl) : ni == 8 ? strip_f64<8, FINE>(excl)
+                                            : ni == 10 ? strip_f64<10, FINE>(excl) : nullptr;
+}
+const void* strip_fn(int precision, int ni, bool excl, long long n) {
+  return n < (precision == kFP32C ? kStripFine32 : kStripFine64) ? strip_fn<true>(precision, ni, excl)
+                                                                 : strip_fn<false>(precision, ni, excl);
 }
 
 // The action sums of every warp's row block.
@@ -702,7 +721,7 @@ cudaError_t configure_strips() {
   for (int prec = 0; prec < 2; ++prec)
     for (int ni : {6, 8, 10, 16})
       for (int v = 0; v < 4 && e == cudaSuccess; ++v)
-        if (const void* fn = strip_fn(prec, ni, (v & 1) != 0, (v & 2) != 0))
+        if (const void* fn = strip_fn(prec, ni, (v & 1) != 0, (v & 2) != 0 ? 0 : 1LL << 40))
           e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)strip_smem(ni));
   return e;
@@ -711,7 +730,7 @@ cudaError_t configure_strips() {
 cudaError_t launch_strips(int precision, const StripPlan& p, double eps2, const IParticles& ip,
                           const JStream& js, const Epilogue& ep, double* scratch, int sms, int mode,
                           double* dst, long long ld, cudaStream_t st) {
-  const void* fn = strip_fn(precision, p.tb, eps2 == 0.0, ip.n < kStripFine64);
+  const void* fn = strip_fn(precision, p.tb, eps2 == 0.0, ip.n);
   if (!fn) return cudaErrorInvalidValue;
   IParticles a0 = ip;
   JStream a1 = js;

@@ -54,3 +54,13 @@ def test_fp64_strips(ctx, nbr, oracle, n, eps2):
 def test_fp64_persistent_run(ctx, nbr, oracle, n):
     run, small = median_errors(ctx, oracle, system(nbr, n, "equal"), FP64, 1e-4, ["run", (1, 8)])
     assert run <= 1.03 * small, (run, small)
+
+
+# FP32C strips against the small-system kernel with 2 lane groups (up to 8192
+# particles) and the large kernel, which served these sizes; 10 % is a third of
+# what one chain of additions per reaction, or one origin per tile, adds
+@pytest.mark.parametrize("n,other", [(6000, (1, 2)), (8192, (1, 2)), (12001, (8, 2))])
+@pytest.mark.parametrize("eps2", [1e-6, 1e-4])
+def test_fp32c_strips(ctx, nbr, oracle, n, other, eps2):
+    strips, before = median_errors(ctx, oracle, system(nbr, n, "spread"), FP32C, eps2, [(3, 8), other])
+    assert strips <= 1.1 * before, (strips, before)
