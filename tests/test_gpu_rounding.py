@@ -64,3 +64,28 @@ def test_fp64_persistent_run(ctx, nbr, oracle, n):
 def test_fp32c_strips(ctx, nbr, oracle, n, other, eps2):
     strips, before = median_errors(ctx, oracle, system(nbr, n, "spread"), FP32C, eps2, [(3, 8), other])
     assert strips <= 1.1 * before, (strips, before)
+
+
+# Masses in whole ratios carry no rounding of their own: a system whose masses are
+# multiples of 1/7000 moves as one of multiples of 2^-13 (exact in 32 bits), up to
+# the roundings of the factor, the sums' product with it and this quotient
+@pytest.mark.parametrize("masses", ["equal", "whole"])
+def test_fp32c_strips_scale_with_the_mass(ctx, nbr, masses):
+    n = 7000
+    s = system(nbr, n, "equal")
+    ratio = np.ones(n) if masses == "equal" else np.random.default_rng(1).choice([1.0, 3.0, 1000.0], n)
+    a = []
+    for unit in (1.0 / 7000, 2.0 ** -13):
+        ctx.upload({"x": s["x"], "y": s["y"], "z": s["z"], "m": unit * ratio})
+        a.append(ctx.forces(FP32C, eps2=1e-6) / unit)
+    assert np.abs(a[0] / a[1] - 1.0).max() <= 1e-15
+
+
+@pytest.mark.parametrize("m0", [0.0, 0.7, 1.99999999, 1e-30, 5e-324])
+def test_fp32c_strips_any_mass_of_particle_0(ctx, nbr, oracle, m0):
+    s = system(nbr, 4500, "spread")
+    s["m"][0] = m0
+    ctx.upload(s)
+    ref = oracle.accel(s["x"], s["y"], s["z"], s["m"], eps2=1e-4, extended=True)
+    e = rel_err(ctx.forces(FP32C, eps2=1e-4), ref)
+    assert np.median(e) <= 1e-6 and e.max() <= 1e-4
