@@ -334,7 +334,8 @@ int nbr_get_force_tiling(nbr_ctx* ctx, int precision, double eps2, int* tile, in
 int nbr_get_force_config(nbr_ctx* ctx, int precision, double eps2, int* ni, int* warps, int* split);
 /* Times the supported configurations for the uploaded system and stores the
  * fastest in the autotune cache file (see nbr_tune_cache_path) under the
- * system's (precision, log2 N, log2 source tiles, eps == 0) bucket: receivers
+ * system's (precision, log2 N, log2 source tiles, eps == 0) bucket (N = 4096
+ * and 4097 .. 8191, where the default becomes Newton-3, are two): receivers
  * per thread and warps per CTA (the i-tile), three j-splits, the small-N and
  * Newton-3 kernels, and, when the large kernel's default configuration wins,
  * its j-tile (64, 128, 256) and unroll depth (2, 4, 8).  Later evaluations in

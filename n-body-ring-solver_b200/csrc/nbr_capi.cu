@@ -221,6 +221,10 @@ std::string lib_dir() {
   return ".";
 }
 
+// Sizes by powers of two.  Where the Newton-3 default begins inside one (at 4097)
+// its part of it has a key of its own (":n3"): a result for a system below it,
+// or an entry from before the default began there, says nothing about the
+// sizes above.
 std::string tune_key(int precision, long long n_i, int ntiles, bool excl) {
   int bucket = 0;
   while ((1LL << (bucket + 1)) <= n_i) ++bucket;
@@ -228,7 +232,7 @@ std::string tune_key(int precision, long long n_i, int ntiles, bool excl) {
   while ((1LL << (jb + 1)) <= (long long)ntiles) ++jb;
   std::ostringstream k;
   k << (precision == kFP32C ? "fp32c" : "fp64") << ":i" << bucket << ":j" << jb
-    << (excl ? ":e0" : "");
+    << (excl ? ":e0" : "") << (n_i >= kN3MinN && (1LL << bucket) < kN3MinN ? ":n3" : "");
   return k.str();
 }
 
@@ -335,7 +339,8 @@ ForceConfig choose_config(nbr_ctx* c, int precision, double eps2, long long n_i,
     // 57.3, 164 / 114; and larger systems, see uses_strips and nbr_strip.cu).
     if (whole && n_i >= kN3MinN && n_i <= kN3MaxN) dflt = ForceConfig{3, kN3Warps, 0};
     else if (F) dflt = ForceConfig{1, F, 0};
-    cfg = it != g_tune->end() ? it->second : dflt;
+    // (a Newton-3 result is of no use to a range or separate sets)
+    cfg = it != g_tune->end() && (whole || it->second.ni != 3) ? it->second : dflt;
   }
   if (cfg.split <= 0) cfg.split = auto_split(precision, eps2, cfg, n_i, ntiles, c->sms);
   // at most one split per ring stage of sources (j-tile: 128 by default)
@@ -1635,7 +1640,9 @@ int nbr_autotune(nbr_ctx* c, int precision, double eps2) {
   float best_ms = 1e30f;
   for (auto& cw : cand) {
     if (cw[0] == 1 && s.n > 65536) continue;  // the small-N kernel only competes on small systems
-    if (cw[0] == 3 && s.n < 8192) continue;
+    // Newton-3 wherever it can be the default; two warps per row block only compete
+    // on larger systems
+    if (cw[0] == 3 && (long long)s.n < (cw[1] == kN3Warps ? kN3MinN : 8192)) continue;
     if (cw[0] == 3 && cw[1] == 16 && precision != kFP32C) continue;  // FP64 has one Newton-3 layout
     ForceConfig base{cw[0], cw[1], 1};
     const int s0 = auto_split(precision, eps2, base, (long long)s.n, s.ntiles, c->sms);

@@ -44,6 +44,33 @@ def test_single_system_autotune(ctx, nbr, oracle):
 
 
 @pytest.mark.parametrize("prec", [FP64, FP32C])
+def test_autotune_where_newton3_begins(ctx, nbr, prec):
+    """The Newton-3 default begins inside a power of two: the strips, half again
+    as fast as any other kernel there, are among the candidates; a system below
+    and separate receiver and source sets keep their own choice."""
+    n, eps2 = 5000, 1e-6
+    s, below = nbr.plummer(n, 8), nbr.plummer(4096, 8)
+
+    def pairs():
+        return ctx.accel_ij(s["x"], s["y"], s["z"], s["x"], s["y"], s["z"], s["m"],
+                            precision=prec, eps2=eps2)
+
+    def config(system):
+        ctx.upload(system)
+        return ctx.get_force_config(prec, eps2)
+
+    default_below, default_pairs = config(below), pairs()
+    ctx.upload(s)
+    ctx.autotune(prec, eps2)
+    assert ctx.get_force_config(prec, eps2)[:2] == (3, 8)
+    assert config(below) == default_below
+    np.testing.assert_array_equal(pairs(), default_pairs)
+    # and the other way round
+    ctx.autotune(prec, eps2)
+    assert config(s)[:2] == (3, 8)
+
+
+@pytest.mark.parametrize("prec", [FP64, FP32C])
 def test_batch_autotune(ctx, nbr, oracle, prec):
     sizes = [40, 130, 300, 513, 1000, 2000, 3000]
     off, st = make_batch(nbr, sizes, seed=12)
