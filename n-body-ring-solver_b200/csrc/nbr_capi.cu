@@ -86,7 +86,7 @@ bool RunKey::operator==(const RunKey& o) const {
       fsal != o.fsal || cur != o.cur || rec_ok[0] != o.rec_ok[0] || rec_ok[1] != o.rec_ok[1] ||
       cfg.ni != o.cfg.ni || cfg.warps != o.cfg.warps || cfg.split != o.cfg.split ||
       cfg.tile != o.cfg.tile || cfg.unroll != o.cfg.unroll ||
-      wait_ns != o.wait_ns || skip_tile != o.skip_tile)
+      wait_ns != o.wait_ns || skip_tile != o.skip_tile || strips != o.strips || bands != o.bands)
     return false;
   for (int i = 0; i < 7; ++i)
     if (ptr[i] != o.ptr[i]) return false;
@@ -447,8 +447,11 @@ StripLaunches strip_launches(nbr_ctx* c, int precision) {
 // evaluation on B200, CTA grid against strips: 32768 812 / 722, 65536 2904 /
 // 2840, 131072 11323 / 11293, 262144 44156 / 44625, 2^20 705 / 718 ms: the
 // strips' 24 B of reactions per (320 rows, particle) take more launches).
+// Test hook: NBR_TEST_N3_GRID set, FP64 takes the CTA grid at any size, so that
+// systems small enough for the oracle reach it.
 bool uses_strips(int precision, const ForceConfig& cfg, long long n) {
-  return cfg.ni == 3 && cfg.warps == kN3Warps && (precision == kFP32C || n <= kStripMaxN64);
+  if (cfg.ni != 3 || cfg.warps != kN3Warps) return false;
+  return precision == kFP32C || (n <= kStripMaxN64 && !std::getenv("NBR_TEST_N3_GRID"));
 }
 
 // Prepares scratch for a force launch of `cfg` over n_i receivers.
@@ -1431,6 +1434,8 @@ int nbr_run(nbr_ctx* c, int precision, int scheme, int order, double dt, size_t 
     key.n = s.n; key.cap = s.cap; key.fsal = fsal; key.cur = s.cur;
     key.rec_ok[0] = s.rec_ok[0]; key.rec_ok[1] = s.rec_ok[1];
     key.cfg = cfg;
+    key.strips = uses_strips(precision, cfg, (long long)s.n);
+    key.bands = forced_bands();
     {
       JStream probe{};
       pipeline_params(probe);

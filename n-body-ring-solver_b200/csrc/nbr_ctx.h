@@ -171,6 +171,8 @@ struct RunKey {
   ForceConfig cfg{0, 0, 0};
   unsigned long long wait_ns = 0;
   int skip_tile = -1;
+  bool strips = false;  // Newton-3: strips (else the CTA grid), and the launches
+  int bands = 0;        // forced by the test hook
   const void* ptr[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   bool operator==(const RunKey& o) const;
 };
