@@ -457,7 +457,14 @@ bool uses_strips(int precision, const ForceConfig& cfg, long long n) {
 // Prepares scratch for a force launch of `cfg` over n_i receivers.
 int prepare_split(nbr_ctx* c, int precision, const ForceConfig& cfg, long long n_pad_i) {
   if (uses_strips(precision, cfg, (long long)c->sys.n)) {  // (the context's whole system only)
-    long long doubles = strip_launches(c, precision).doubles;
+    const StripLaunches L = strip_launches(c, precision);
+    const StripKernel k{precision, L.ni, (long long)c->sys.n};
+    if (!(k == c->strip_ready)) {
+      const cudaError_t e = prepare_strips(precision, k.n, k.ni);
+      if (e != cudaSuccess) return cuda_fail(c, e, "Newton-3 kernel setup");
+      c->strip_ready = k;
+    }
+    long long doubles = L.doubles;
     cudaError_t e = c->scr.need_part((size_t)doubles);
     if (e == cudaErrorMemoryAllocation && doubles > kN3SliceMaxDoubles &&
         c->strip_single > kN3SliceMaxDoubles) {
@@ -883,7 +890,6 @@ int nbr_ctx_create(int device, nbr_ctx** out) {
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
   if (e == cudaSuccess) e = dalloc((void**)&c->d_err, sizeof(int) * 4);
   if (e == cudaSuccess) e = configure_kernels();
-  if (e == cudaSuccess) e = configure_strips();
   if (e != cudaSuccess) {
     int rc = cuda_fail(nullptr, e, "context setup");
     nbr_ctx_destroy(c);

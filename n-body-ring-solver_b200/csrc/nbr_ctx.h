@@ -176,6 +176,14 @@ struct RunKey {
   const void* ptr[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   bool operator==(const RunKey& o) const;
 };
+// What decides the kernels of an evaluation in strips (but for the softening).
+struct StripKernel {
+  int precision = -1, ni = 0;
+  long long n = 0;
+  bool operator==(const StripKernel& o) const {
+    return precision == o.precision && ni == o.ni && n == o.n;
+  }
+};
 // A captured nbr_run graph, replayed while the key matches.
 constexpr int kRunGraphs = 4;
 struct RunGraph {
@@ -215,6 +223,7 @@ struct nbr_ctx {
   // Most scratch of an evaluation in strips that runs as one launch, lowered
   // when that much could not be allocated, until the next upload.
   long long strip_single = nbr::kN3SingleMaxDoubles;
+  nbr::StripKernel strip_ready;  // the last kernels whose attributes were set
   // The last persistent launch configuration whose attributes were set, and its
   // resident CTAs per SM.
   const void* persist_fn = nullptr;

@@ -265,7 +265,10 @@ std::vector<int> strip_bands(int precision, long long n, int sms, int ni, int ba
 cudaError_t launch_strips(int precision, const StripPlan& p, double eps2, const IParticles& ip,
                           const JStream& js, const Epilogue& ep, double* scratch, int sms, int mode,
                           double* dst, long long ld, cudaStream_t stream);
-cudaError_t configure_strips();
+// Sets the shared memory of the kernels that evaluate a system of n particles,
+// outside stream capture and before their first launch.  (Setting all when a
+// context is created loaded 24 kernels that it might never run: 3 of 30 ms.)
+cudaError_t prepare_strips(int precision, long long n, int ni);
 // Sums of m_i m_j / r over the unordered pairs of the particles, over
 // kInvDistScale, one per strip: at most kEnergyStrips x sms, the number used
 // into *count.  n up to kEnergyMaxN (32-bit unit numbers).

@@ -732,14 +732,14 @@ cudaError_t launch_energy(long long n, double eps2, const IParticles& ip, const 
   return cudaGetLastError();
 }
 
-cudaError_t configure_strips() {
+cudaError_t prepare_strips(int precision, long long n, int ni) {
   cudaError_t e = cudaSuccess;
-  for (int prec = 0; prec < 2; ++prec)
-    for (int ni : {6, 8, 10, 16})
-      for (int v = 0; v < 4 && e == cudaSuccess; ++v)
-        if (const void* fn = strip_fn(prec, ni, (v & 1) != 0, (v & 2) != 0 ? 0 : 1LL << 40))
-          e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)strip_smem(ni));
+  for (bool excl : {false, true}) {
+    const void* fn = strip_fn(precision, ni, excl, n);
+    if (!fn) return cudaErrorInvalidValue;
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)strip_smem(ni));
+  }
   return e;
 }
 
