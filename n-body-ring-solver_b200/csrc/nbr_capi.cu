@@ -328,9 +328,13 @@ ForceConfig choose_config(nbr_ctx* c, int precision, double eps2, long long n_i,
     // FP64 has twice the registers per receiver and prefers 4 per thread.
     ForceConfig dflt = precision == kFP32C ? ForceConfig{8, 2, 0} : ForceConfig{4, 4, 0};
     // Small systems, receiver ranges and separate sets: the warp-splitting
-    // kernel.  Lane groups per warp from a B200 sweep (forces per call, N = 256
-    // .. 262144): FP32C 8 up to 4096 receivers, 2 up to 8192; FP64 8 up to
-    // 16384, 4 up to 32768; above that the large kernels win.
+    // kernel.  Lane groups per warp from a B200 sweep: FP32C 8 up to 4096
+    // receivers, 2 up to 8192; FP64 8 up to 16384, 4 up to 32768.  Ranges and
+    // separate sets of 8192 to 32768 receivers went to the large kernels before
+    // inv_cube; with it, us per FP64 evaluation of n receivers and n sources, this
+    // kernel / the large one: 8192 82 / 104, 12288 165 / 185, 16384 277 / 302, 24576 611 /
+    // 658, 32768 1058 / 1123; with 262144 sources 16384 4176 / 4321, 32768 8239 /
+    // 8472.  (Above it the large kernel is at most 4 % slower, up to 65536.)
     const int F = precision == kFP32C ? (n_i <= 4096 ? 8 : n_i <= 8192 ? 2 : 0)
                                       : (n_i <= 16384 ? 8 : n_i <= 32768 ? 4 : 0);
     // From there to 2^23 particles: Newton-3 (B200, us per KDK step, the best
