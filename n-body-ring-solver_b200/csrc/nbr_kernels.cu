@@ -1801,19 +1801,7 @@ bool force_config_supported(int precision, const ForceConfig& c) {
 
 int force_blocks_per_sm(int precision, double eps2, const ForceConfig& c) {
   int nb = 0;
-  if (c.ni == 3) {
-    const bool ex = eps2 == 0.0;
-    const bool w2 = precision == kFP32C && c.warps == kN3W2Warps;
-    const void* fn = precision == kFP32C
-                         ? (w2 ? (ex ? (const void*)k_force_n3_f32c_w2<true> : (const void*)k_force_n3_f32c_w2<false>)
-                               : (ex ? (const void*)k_force_n3_f32c<true> : (const void*)k_force_n3_f32c<false>))
-                         : (ex ? (const void*)k_force_n3_f64<true> : (const void*)k_force_n3_f64<false>);
-    const int threads = n3_cta_warps(precision, c.warps) * 32;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, threads, n3_smem_bytes(precision, c.warps)) !=
-        cudaSuccess)
-      nb = 0;
-    return nb;
-  }
+  if (c.ni == 3) return 1;  // strips and CTA grid: their registers fill an SM
   const size_t smem = force_smem_bytes(precision, c);
   const bool ex = (eps2 == 0.0);
   if (c.ni == 1) {
@@ -1941,7 +1929,6 @@ double n3_makespan(long long nb, int cols, int sms) {
 
 int n3_cols(long long nb) { return n3_cols_for(nb, device_sms()); }
 int n3_slice_cols(long long nb, int V) { return n3_slice_cols_for(nb, V, device_sms()); }
-double n3_grid_efficiency(long long nb) { return n3_grid_efficiency_for(nb, device_sms()); }
 
 int n3_cols_for(long long nb, int sms) {
   if (nb <= 1) return 1;
@@ -2029,7 +2016,7 @@ double n3_grid_efficiency_for(long long nb, int sms) {
   if (sms < 1) sms = 1;
   const int cols = n3_cols_for(nb, sms);  // before taking the lock (it has its own)
   static std::mutex mu;
-  static std::map<std::pair<long long, int>, double> memo;  // the choice runs per evaluation
+  static std::map<std::pair<long long, int>, double> memo;
   std::lock_guard<std::mutex> lock(mu);
   const auto key = std::make_pair(nb, sms);
   const auto it = memo.find(key);

@@ -142,12 +142,10 @@ void n3_cta_costs(long long nb, int cols, std::vector<double>& cost);
 double n3_makespan(long long nb, int cols, int sms);
 // That launch order: order[launch index] = group-major CTA index.
 void n3_launch_order(long long nb, int cols, std::vector<int>& order);
-// The model's efficiency of the whole-system Newton-3 grid for nb blocks on
-// the current device: the pair work spread evenly over the SMs divided by the
-// grid's finishing time (1 at best).  A host function.
-double n3_grid_efficiency(long long nb);
-// n3_cols, n3_slice_cols and n3_grid_efficiency for a device of `sms` SMs
-// (host functions; no device needed).
+// n3_cols and n3_slice_cols for a device of `sms` SMs, and the model's efficiency
+// of the whole-system grid there: the pair work spread evenly over the SMs
+// divided by the grid's finishing time, 1 at best (host functions; no device
+// needed).
 int n3_cols_for(long long nb, int sms);
 int n3_slice_cols_for(long long nb, int V, int sms);
 double n3_grid_efficiency_for(long long nb, int sms);
