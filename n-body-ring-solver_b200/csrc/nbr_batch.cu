@@ -935,8 +935,8 @@ __global__ void __launch_bounds__(128) k_batch_n3_reduce(const BatchParams p, co
   }
 }
 
-// The state without the systems' padding: one warp per tile copies its real
-// particles of the six arrays to their caller's places.
+// Arrays of the state without the systems' padding: one warp per tile and array
+// (blockIdx.y) copies its real particles to their caller's places.
 struct BatchRows {
   const double* src[6];
 };
@@ -955,9 +955,9 @@ __global__ void __launch_bounds__(128)
   }
   const long long to = off[lo] + (first - poff[lo]);
   const int count = (int)min((long long)kTile, off[lo + 1] - to);
-#pragma unroll
-  for (int f = 0; f < 6; ++f)
-    for (int k = lane; k < count; k += 32) dst[f * n_real + to + k] = rows.src[f][first + k];
+  const double* src = rows.src[blockIdx.y];
+  dst += blockIdx.y * n_real;
+  for (int k = lane; k < count; k += 32) dst[to + k] = src[first + k];
 }
 
 // Per-system diagnostics: one CTA per system.  out[s * 9 + c] =
@@ -1442,26 +1442,32 @@ int nbr_batch_download(nbr_ctx* c, double* x, double* y, double* z, double* vx, 
   cudaError_t e = cudaSuccess;
   const int a = b.s.cur;
   double* out[6] = {x, y, z, vx, vy, vz};
-  if (!b.d_flat && dalloc((void**)&b.d_flat, 6 * b.n_real * sizeof(double)) != cudaSuccess) {
+  const double* src[6] = {b.s.pos[a][0], b.s.pos[a][1], b.s.pos[a][2],
+                          b.s.vel[0], b.s.vel[1], b.s.vel[2]};
+  // all arrays at once where they are small (a launch each took 20 of 300 us),
+  // else through one array's copy
+  const int per = stage_fits(6 * b.n_real) ? 6 : 1;
+  if (!b.d_flat && dalloc((void**)&b.d_flat, per * b.n_real * sizeof(double)) != cudaSuccess) {
     // no room on the device: the padding is taken out on the host
     cudaGetLastError();
-    b.d_flat = nullptr;
-    const double* src[6] = {b.s.pos[a][0], b.s.pos[a][1], b.s.pos[a][2],
-                            b.s.vel[0], b.s.vel[1], b.s.vel[2]};
     std::vector<double> h;
     for (int f = 0; f < 6; ++f)
       if (out[f] && e == cudaSuccess) e = fetch_padded(c, h, out[f], src[f]);
     return e == cudaSuccess ? NBR_OK : cuda_fail(c, e, "batch download");
   }
-  const BatchRows rows{{b.s.pos[a][0], b.s.pos[a][1], b.s.pos[a][2], b.s.vel[0], b.s.vel[1], b.s.vel[2]}};
   const long long ntiles = b.poff[b.nsys] / kTile;
-  k_batch_flatten<<<(unsigned)((ntiles + 3) / 4), 128, 0, c->stream>>>(
-      rows, b.d_flat, (long long)b.n_real, b.d_poff, b.d_off, (int)b.nsys, ntiles);
-  e = cudaGetLastError();
-  for (int f = 0; f < 6; ++f)
+  for (int f = 0; f < 6; ++f) {
+    if (e == cudaSuccess && f % per == 0 && (per > 1 || out[f])) {
+      BatchRows rows{};
+      for (int k = 0; k < per; ++k) rows.src[k] = src[f + k];
+      k_batch_flatten<<<dim3((unsigned)((ntiles + 3) / 4), per), 128, 0, c->stream>>>(
+          rows, b.d_flat, (long long)b.n_real, b.d_poff, b.d_off, (int)b.nsys, ntiles);
+      e = cudaGetLastError();
+    }
     if (out[f] && e == cudaSuccess)
-      e = cudaMemcpyAsync(out[f], b.d_flat + f * b.n_real, b.n_real * sizeof(double),
+      e = cudaMemcpyAsync(out[f], b.d_flat + f % per * b.n_real, b.n_real * sizeof(double),
                           cudaMemcpyDeviceToHost, c->stream);
+  }
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   return e == cudaSuccess ? NBR_OK : cuda_fail(c, e, "batch download");
 }

@@ -65,7 +65,7 @@ struct BatchState {
   long long* d_poff = nullptr;       // padded offsets (device), nsys + 1
   int* d_nreal = nullptr;            // real size of each system (device)
   long long* d_off = nullptr;        // real offsets (device), nsys + 1
-  double* d_flat = nullptr;          // [6][n_real]: the state without padding (first download)
+  double* d_flat = nullptr;          // one array, or six small ones, without padding (first download)
   int* d_sys_of_tile = nullptr;      // system index of every padded tile
   // Work queues of (system | kWideItem flag, first receiver tile), cost
   // ordered: [0] one-tile items only, [1] two-tile items where a system has

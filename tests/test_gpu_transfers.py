@@ -85,6 +85,29 @@ def test_batch_download_is_the_upload(ctx, nbr):
         np.testing.assert_array_equal(got[k], st[k])
 
 
+def test_batch_download_keeps_one_array(nbr):
+    """What a download allocates and keeps is one array without padding, whichever
+    arrays are asked for."""
+    torch = pytest.importorskip("torch")
+    sizes = np.full(64, 32700)
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    n = int(off[-1])
+    rng = np.random.default_rng(2)
+    st = {k: np.abs(rng.standard_normal(n)) for k in nbr.KEYS}
+    with nbr.Context(0) as c:
+        c.batch_upload(off, st)
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        z, vx = np.zeros(n), np.zeros(n)
+        assert c.L.nbr_batch_download(c.h, None, None, nbr._p(z), nbr._p(vx), None, None) == 0
+        np.testing.assert_array_equal(z, st["z"])
+        np.testing.assert_array_equal(vx, st["vx"])
+        got = c.batch_download()
+        for k in ("x", "y", "z", "vx", "vy", "vz"):
+            np.testing.assert_array_equal(got[k], st[k])
+        assert free - torch.cuda.mem_get_info()[0] <= 8 * n + (4 << 20)  # allocation granularity
+
+
 # Where there is no room for what a transfer or a launch would take at its
 # fastest, the call does without it: the same results.
 def failing_allocation(monkeypatch, call, k="1"):
