@@ -1129,8 +1129,12 @@ int batch_grid(nbr_ctx* c, int prec, double eps2) {
   BatchState::N3List& l3 = b.n3[pi];
   if (wi == 2 && l3.slots > 0 && !l3.d_rea) {
     cudaError_t e = cudaSuccess;
-    if (!b.d_act) e = dalloc((void**)&b.d_act, 3 * b.s.n_pad * sizeof(double));
-    if (e == cudaSuccess) e = dalloc((void**)&l3.d_rea, (size_t)l3.slots * 3 * kTile * sizeof(double));
+    if (!b.d_act)
+      e = with_room(c, [&] { return dalloc((void**)&b.d_act, 3 * b.s.n_pad * sizeof(double)); });
+    if (e == cudaSuccess)
+      e = with_room(c, [&] {
+        return dalloc((void**)&l3.d_rea, (size_t)l3.slots * 3 * kTile * sizeof(double));
+      });
     if (e != cudaSuccess) {
       dfree(l3.d_rea);
       l3.d_rea = nullptr;
@@ -1277,7 +1281,7 @@ int nbr_batch_upload(nbr_ctx* c, size_t nsys, const size_t* offsets, const doubl
   }
   b.pairs_per_eval = pairs;
   const size_t np = (size_t)b.poff[nsys];
-  cudaError_t e = b.s.reserve(np);
+  cudaError_t e = with_room(c, [&] { return b.s.reserve(np); });
   if (e != cudaSuccess) {
     b.release();  // no half-built batch is left behind
     return cuda_fail(c, e, "batch allocation");

@@ -98,6 +98,17 @@ void RunGraph::release() {
   *this = RunGraph();
 }
 
+bool give_back(nbr_ctx* c) {
+  bool any = c->bat.d_flat != nullptr;
+  dfree(c->bat.d_flat);
+  c->bat.d_flat = nullptr;
+  for (RunGraph& g : c->run_graph) {
+    any |= g.exec != nullptr;
+    g.release();
+  }
+  return any;
+}
+
 bool finite_array(const double* a, size_t n) {
   bool ok = true;
   for (size_t i = 0; i < n; ++i) ok &= std::isfinite(a[i]);
@@ -469,14 +480,14 @@ int prepare_split(nbr_ctx* c, int precision, const ForceConfig& cfg, long long n
       c->strip_ready = k;
     }
     long long doubles = L.doubles;
-    cudaError_t e = c->scr.need_part((size_t)doubles);
+    cudaError_t e = with_room(c, [&] { return c->scr.need_part((size_t)doubles); });
     if (e == cudaErrorMemoryAllocation && doubles > kN3SliceMaxDoubles &&
         c->strip_single > kN3SliceMaxDoubles) {
       // No room for one launch's scratch (up to 9 GiB; the CTA grid, which
-      // took 0.6 of it, may have found room): several launches of 2 GiB.  A
-      // graph captured with the larger scratch must not run on the smaller.
+      // took 0.6 of it, may have found room): several launches of 2 GiB.  (No
+      // graph captured with the larger scratch is left to run on the smaller.)
       cudaGetLastError();
-      for (RunGraph& g : c->run_graph) g.release();
+      give_back(c);
       c->strip_single = kN3SliceMaxDoubles;
       doubles = strip_launches(c, precision).doubles;
       e = c->scr.need_part((size_t)doubles);
@@ -490,13 +501,15 @@ int prepare_split(nbr_ctx* c, int precision, const ForceConfig& cfg, long long n
     long long acc_off = 0;
     const long long need =
         V == 1 ? n3_scratch_doubles(nb) : n3_banded_doubles(nb, V, (long long)c->sys.n_pad, &acc_off);
-    cudaError_t e = c->scr.need_part((size_t)need);
+    cudaError_t e = with_room(c, [&] { return c->scr.need_part((size_t)need); });
     if (e == cudaSuccess && V == 1) e = n3_order_prepare(c, nb);
     return e == cudaSuccess ? NBR_OK : cuda_fail(c, e, "Newton-3 scratch");
   }
   if (cfg.split <= 1) return NBR_OK;
-  cudaError_t e = c->scr.need_part((size_t)cfg.split * 3 * (size_t)n_pad_i);
-  if (e == cudaSuccess) e = c->scr.need_counters((size_t)(n_pad_i / 64 + 1));
+  cudaError_t e =
+      with_room(c, [&] { return c->scr.need_part((size_t)cfg.split * 3 * (size_t)n_pad_i); });
+  if (e == cudaSuccess)
+    e = with_room(c, [&] { return c->scr.need_counters((size_t)(n_pad_i / 64 + 1)); });
   return e == cudaSuccess ? NBR_OK : cuda_fail(c, e, "split scratch");
 }
 
@@ -743,7 +756,7 @@ int potential_system(nbr_ctx* c, double G, double eps2, double* dphi, size_t red
   pipeline_params(js);
   NBR_CHECKED_ONLY(ip.len = (long long)(s.cap + kRangeSlack); js.len = (long long)s.cap;)
   if (!dphi && (long long)s.n <= kEnergyMaxN) {
-    cudaError_t e = c->scr.need_red(red_off + potential_sums(c) + 16);
+    cudaError_t e = with_room(c, [&] { return c->scr.need_red(red_off + potential_sums(c) + 16); });
     if (e != cudaSuccess) return cuda_fail(c, e, "potential scratch");
     double* sums = c->scr.red + red_off;
     int strips = 0;
@@ -763,7 +776,7 @@ int potential_system(nbr_ctx* c, double G, double eps2, double* dphi, size_t red
   if (rc) return rc;
   const long long chunk = 32LL * kPotNI * kPotWarps;
   const int chunks = (int)(((long long)s.n + chunk - 1) / chunk);
-  cudaError_t e = c->scr.need_red(red_off + (size_t)chunks + 16);
+  cudaError_t e = with_room(c, [&] { return c->scr.need_red(red_off + (size_t)chunks + 16); });
   if (e != cudaSuccess) return cuda_fail(c, e, "potential scratch");
   PotentialOut po{};
   po.G = G;
@@ -791,7 +804,7 @@ int diag_system(nbr_ctx* c, double G, double eps2, nbr_diag* out) {
   // moments (8 x nb), their sums (16), then the potential's sums and U, then
   // the results packed: sized once here so that nothing below reallocates.
   const size_t used = (size_t)nb * 9 + 32 + potential_sums(c);
-  cudaError_t e = c->scr.need_red(used + 16);
+  cudaError_t e = with_room(c, [&] { return c->scr.need_red(used + 16); });
   if (e != cudaSuccess) return cuda_fail(c, e, "diag scratch");
   double* part = c->scr.red;
   double* res = c->scr.red + (size_t)nb * 8;
@@ -945,7 +958,7 @@ int nbr_system_upload(nbr_ctx* c, size_t n, const double* x, const double* y, co
   cudaSetDevice(c->device);
   SysState& s = c->sys;
   const size_t cap0 = s.cap;
-  cudaError_t e = s.reserve(n);
+  cudaError_t e = with_room(c, [&] { return s.reserve(n); });
   if (s.cap != cap0)  // their buffers are gone
     for (RunGraph& g : c->run_graph) g.release();
   if (e != cudaSuccess) return cuda_fail(c, e, "system allocation");
@@ -1153,7 +1166,7 @@ int nbr_n3_slice_accel(nbr_ctx* c, int precision, double eps2, int slice_begin, 
   if (e != cudaSuccess) return cuda_fail(c, e, "pack");
   const long long nb = ((long long)s.n + kN3Block - 1) / kN3Block;
   const long long need = n3_slices_scratch_doubles(nb, slice_begin, slice_end, nslices);
-  e = c->scr.need_part((size_t)std::max<long long>(need, 1));
+  e = with_room(c, [&] { return c->scr.need_part((size_t)std::max<long long>(need, 1)); });
   if (e != cudaSuccess) return cuda_fail(c, e, "Newton-3 slice scratch");
   ForceConfig cfg = choose_config(c, precision, eps2, (long long)s.n, s.ntiles);
   const int warps = cfg.ni == 3 ? cfg.warps : kN3Warps;
@@ -1270,7 +1283,7 @@ int nbr_accel_ij(nbr_ctx* c, int precision, size_t n_i, const double* xi, const 
   // Receivers live in ij.pos[0] (+ mass), sources in ij.pos[1] (+ j_mass).
   SysState& r = c->ij;
   const size_t nmax = std::max(n_i, n_j);
-  cudaError_t e = r.reserve(nmax);
+  cudaError_t e = with_room(c, [&] { return r.reserve(nmax); });
   if (e != cudaSuccess) return cuda_fail(c, e, "ij allocation");
   const long long npi = (long long)(((n_i + 1023) / 1024) * 1024);
   const long long npj = (long long)(((n_j + 1023) / 1024) * 1024);
@@ -1518,8 +1531,13 @@ int nbr_run(nbr_ctx* c, int precision, int scheme, int order, double dt, size_t 
         s.rec_ok[1] = rec1;
         return rc != NBR_OK ? rc : cuda_fail(c, ee, "end capture");
       }
+      long long kept = kernels;
+      for (int k = 1; k < kRunGraphs; ++k) {
+        kept += c->run_graph[k].kernels;
+        if (k >= 2 && kept > kRunGraphKernels) c->run_graph[k].release();
+      }
       cudaGraphExec_t exec = nullptr;
-      e = cudaGraphInstantiate(&exec, graph, 0);
+      e = with_room(c, [&] { return cudaGraphInstantiate(&exec, graph, 0); });
       cudaGraphDestroy(graph);
       if (e != cudaSuccess) {
         s.cur = cur0;

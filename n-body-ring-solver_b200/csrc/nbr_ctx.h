@@ -126,6 +126,19 @@ int fail(nbr_ctx* c, int code, const std::string& msg);
 int cuda_fail(nbr_ctx* c, cudaError_t e, const char* where);
 cudaError_t dalloc(void** p, size_t bytes);
 void dfree(void* p);
+// Gives back what a context keeps for speed alone: the graphs of nbr_run and the
+// batch's copy without padding.  False if there was nothing.
+bool give_back(nbr_ctx* c);
+// alloc(), and where it finds no room once more with that given back.
+template <class F>
+cudaError_t with_room(nbr_ctx* c, F alloc) {
+  cudaError_t e = alloc();
+  if (e == cudaErrorMemoryAllocation && give_back(c)) {
+    cudaGetLastError();
+    e = alloc();
+  }
+  return e;
+}
 bool finite_array(const double* a, size_t n);
 int check_device_error(nbr_ctx* c);
 // The status of a device error word already on the host (0: NBR_OK).
@@ -184,8 +197,11 @@ struct StripKernel {
     return precision == o.precision && ni == o.ni && n == o.n;
   }
 };
-// A captured nbr_run graph, replayed while the key matches.
+// A captured nbr_run graph, replayed while the key matches.  The last two stay; the
+// two before them only while all hold at most kRunGraphKernels launches (2.5 KB of
+// device and 6.6 KB of host memory each).
 constexpr int kRunGraphs = 4;
+constexpr int kRunGraphKernels = 16384;
 struct RunGraph {
   cudaGraphExec_t exec = nullptr;
   RunKey key;

@@ -165,3 +165,35 @@ def test_download_leaves_a_pending_error(nbr, monkeypatch):
         with pytest.raises(nbr.NbrError):
             c.synchronize()
         assert np.isfinite(c.forces(FP64, eps2=1e-4)).all()
+
+
+def test_graphs_give_way(nbr, oracle, monkeypatch):
+    """What a context keeps for speed is given back where an allocation fails."""
+    small, large = nbr.plummer(4500, 5), nbr.plummer(9000, 6)
+    for keep in ("graph", "batch copy"):
+        with nbr.Context(0) as c:
+            if keep == "graph":
+                c.upload(small)
+                c.run(FP64, nbr.KDK, 2, 1e-4, 2, eps2=1e-4)
+            else:
+                c.batch_upload(np.array([0, 4000, 4500]), small)
+                c.batch_download()
+            failing_allocation(monkeypatch, lambda: c.upload(large))
+            ref = oracle.accel(large["x"], large["y"], large["z"], large["m"], eps2=1e-4, extended=True)
+            assert rel_err(c.forces(FP64, eps2=1e-4), ref).max() <= 1e-12
+            if keep == "batch copy":
+                np.testing.assert_array_equal(c.batch_download()["x"], small["x"])
+
+
+def test_long_graphs_are_not_all_kept(nbr):
+    """Two graphs stay, of whatever length; more only while they are short."""
+    torch = pytest.importorskip("torch")
+    free = []
+    with nbr.Context(0) as c:
+        c.upload(nbr.plummer(4500, 5))
+        for steps in (6000, 6001, 6002, 6003):  # about 12000 launches, 30 MB each
+            c.run(FP64, nbr.EULER, 2, 1e-9, steps, eps2=1e-2)
+            torch.cuda.synchronize()
+            free.append(torch.cuda.mem_get_info()[0])
+    assert free[0] - free[1] > 16 << 20
+    assert free[1] - free[3] <= 16 << 20
