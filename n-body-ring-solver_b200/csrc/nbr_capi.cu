@@ -349,9 +349,9 @@ ForceConfig choose_config(nbr_ctx* c, int precision, double eps2, long long n_i,
     const int F = precision == kFP32C ? (n_i <= 4096 ? 8 : n_i <= 8192 ? 2 : 0)
                                       : (n_i <= 16384 ? 8 : n_i <= 32768 ? 4 : 0);
     // From there to 2^23 particles: Newton-3 (B200, us per KDK step, the best
-    // kernel above against the strips: FP32C 4608 33.6 / 17.8, 6000 42.6 / 22.4,
-    // 8192 53.6 / 33.4, 12001 108.6 / 61.9; FP64 36.7 / 27.9, 56.1 / 34.7, 87.8 /
-    // 57.3, 164 / 114; and larger systems, see uses_strips and nbr_strip.cu).
+    // kernel above against the strips: FP32C 6000 42.6 / 20.8, 8192 53.6 / 32.0,
+    // 12001 108.6 / 58.5; FP64 56.1 / 33.2, 87.8 / 55.0, 164 / 111; and larger
+    // systems, see uses_strips and nbr_strip.cu).
     if (whole && n_i >= kN3MinN && n_i <= kN3MaxN) dflt = ForceConfig{3, kN3Warps, 0};
     else if (F) dflt = ForceConfig{1, F, 0};
     // (a Newton-3 result is of no use to a range or separate sets)
@@ -459,8 +459,8 @@ StripLaunches strip_launches(nbr_ctx* c, int precision) {
   return L;
 }
 // FP32C: every whole system.  FP64: up to kStripMaxN64 particles (us per
-// evaluation on B200, CTA grid against strips: 32768 812 / 722, 65536 2904 /
-// 2840, 131072 11323 / 11293, 262144 44156 / 44625, 2^20 705 / 718 ms: the
+// evaluation on B200, CTA grid against strips: 32768 812 / 719, 65536 2904 /
+// 2828, 131072 11323 / 11293, 262144 44156 / 44625, 2^20 705 / 718 ms: the
 // strips' 24 B of reactions per (320 rows, particle) take more launches).
 // Test hook: NBR_TEST_N3_GRID set, FP64 takes the CTA grid at any size, so that
 // systems small enough for the oracle reach it.

@@ -125,7 +125,7 @@ __device__ __forceinline__ double inv_cube(double r2) {
 // the next term below 5/16 (1.9e-6)^3 = 2.1e-18; 20/9 and 3/8 are rounded to
 // the doubles whose product is nearest 1 at h = 0 (2e-17).  Four FP64
 // operations and one MUFU.  Only for normal r2: a caller whose sums stay
-// finite where r2 is subnormal takes rsqrt() there (see tiny_r2).
+// finite where r2 is subnormal takes inv_dist_tiny there (r2 below kTinyHi).
 constexpr double kInvDistScale = 0.37499999999999994;
 __device__ __forceinline__ double inv_dist(double r2) {
   const double y = rsqrt_seed64(r2);

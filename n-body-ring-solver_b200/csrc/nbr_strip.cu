@@ -26,8 +26,8 @@
 // 16384 particles, and its warps meet at a barrier per tile.  Strips write
 // one reaction per (row block, particle) instead of one per (2048 rows,
 // particle), 12 B (FP32C) or 24 B (FP64): at N = 262144 0.8 and 2.6 GB, written
-// during the loop and read once.  us per evaluation on B200 (KDK run; before,
-// after): see strip_choose.
+// during the loop and read once.  Both forms' times stand where the choice between
+// them is made, at choose_config and uses_strips (nbr_capi.cu).
 #include "nbr_device.cuh"
 #include "nbr_kernels.cuh"
 
@@ -74,9 +74,9 @@ __device__ inline int strip_row(const StripPlan& p, int u) {
 // serialization: a kernel may be set up while the one before it in the stream
 // finishes.  It reads nothing that a kernel writes and writes nothing before
 // grid_dependency_wait(), which returns when that kernel has completed and its
-// writes are visible.  us per
-// evaluation in a graph, without / with: FP64 N = 4224 23.9 / 21.3, 6000 34.7 / 33.6;
-// FP32C 4224 18.4 / 15.4, 6000 22.4 / 21.2, 12001 61.9 / 59.7.
+// writes are visible.  us per evaluation in a graph, without / with: FP64 N = 4224
+// 23.9 / 21.3, 6000 34.7 / 33.6; FP32C 4224 18.4 / 15.4, 6000 22.4 / 21.2, 12001 61.9 /
+// 59.7.
 __device__ __forceinline__ void grid_dependency_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
@@ -535,6 +535,8 @@ __global__ void __launch_bounds__(kStripWarps * 32, NI == 4 ? 2 : 1)
 // 15.6 / 15.5 / 16.4, 12001 61.1 / 60.1 / 58.1, 65536 1385 / 1375 / 1366, 262144
 // 21743 / 21576 / 21510; FP64 4224 21.4 / 21.1 / 22.0, 12001 112.4 / 112.4 / 110.1,
 // 16000 180.6 / 181.9 / 181.2, 196608 25214 / 25072 / 25042.
+// The last sums by halves, a warp per axis, instead of one warp in order: FP64 4224 21.2 /
+// 20.8, 12001 110.3 / 111.0.
 constexpr int kRedWarps = 16;
 
 template <int PREC, int PER_SM>
