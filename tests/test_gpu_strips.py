@@ -153,3 +153,16 @@ def test_energy_of_an_extreme_pair(ctx, d):
     # a coincident pair is skipped without softening
     ctx.upload({"x": z, "y": z, "z": z, "m": np.array([0.5, 0.5])})
     assert ctx.diagnostics()["U"] == 0.0 and ctx.potential(per_particle=True)[0] == 0.0
+
+
+# Where the reactions' form changes (FP64 12288, FP32C 131072 particles), ragged too
+@pytest.mark.parametrize("prec,n", [(FP64, 12287), (FP64, 12288), (FP64, 12289),
+                                    (FP32C, 131071), (FP32C, 131072), (FP32C, 131073)])
+@pytest.mark.parametrize("eps2", [0.0, 1e-6])
+def test_reactions_where_their_form_changes(ctx, nbr, oracle, prec, n, eps2):
+    s = nbr.plummer(n, n)
+    ctx.upload(s)
+    assert ctx.get_force_config(prec, eps2)[0] == 3
+    idx = np.unique(np.concatenate([np.linspace(0, n - 1, 300).astype(int), np.arange(n - 3, n)]))
+    ref = oracle.accel_subset(s["x"], s["y"], s["z"], s["m"], idx, eps2=eps2)
+    check(ctx.forces(prec, eps2=eps2)[:, idx], ref, prec)
