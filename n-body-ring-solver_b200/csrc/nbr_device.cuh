@@ -149,6 +149,17 @@ __device__ __forceinline__ double sum_by_halves(const double* p, int ld) {
   else return sum_by_halves<K / 2>(p, ld) + sum_by_halves<K / 2>(p + K / 2 * ld, ld);
 }
 
+// hi + lo <- hi + lo + x: the rounding error of the sum goes to lo (Knuth TwoSum).
+__device__ __forceinline__ void add_error_free(double& hi, double& lo, double x) {
+  const double s = hi + x, b = s - hi;
+  lo += (hi - (s - b)) + (x - b);
+  hi = s;
+}
+// scale (hi + lo), rounded once; where hi overflowed, its infinity (lo is NaN).
+__device__ __forceinline__ double scaled_sum(double scale, double hi, double lo) {
+  return isfinite(hi) ? fma(scale, hi, scale * lo) : scale * hi;
+}
+
 // Knuth TwoSum of the packed pair (hi + p): hi <- rounded sum, lo += the
 // rounding error.  Six packed adds; exact error term for round-to-nearest.
 __device__ __forceinline__ void two_sum2(u64& hi, u64& lo, u64 p) {

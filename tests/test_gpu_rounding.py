@@ -89,3 +89,32 @@ def test_fp32c_strips_any_mass_of_particle_0(ctx, nbr, oracle, m0):
     ref = oracle.accel(s["x"], s["y"], s["z"], s["m"], eps2=1e-4, extended=True)
     e = rel_err(ctx.forces(FP32C, eps2=1e-4), ref)
     assert np.median(e) <= 1e-6 and e.max() <= 1e-4
+
+
+def potentials(s, eps2, idx):
+    """Extended-precision potentials of the particles idx."""
+    x = np.stack([s[k] for k in "xyz"]).astype(np.longdouble)
+    m = s["m"].astype(np.longdouble)
+    out = np.zeros(len(idx), np.longdouble)
+    for k, i in enumerate(idx):
+        d = x - x[:, i:i + 1]
+        r2 = (d * d).sum(0) + np.longdouble(eps2)
+        r2[i] = 1
+        w = m / np.sqrt(r2)
+        w[i] = 0
+        out[k] = -w.sum()
+    return out
+
+
+# rms errors of a potential in the kernel with rsqrt(double): no more than these
+@pytest.mark.parametrize("n,before", [(2048, 1.78e-16), (6000, 1.62e-16)])
+def test_potentials(ctx, nbr, n, before):
+    e = []
+    for seed in range(4):
+        s = nbr.plummer(n, seed)
+        ctx.upload(s)
+        idx = np.arange(0, n, max(1, n // 500))
+        ref = potentials(s, 1e-4, idx)
+        got = ctx.potential(eps2=1e-4, per_particle=True)[1][idx]
+        e.append(((got - ref) / ref).astype(float))
+    assert np.sqrt(np.mean(np.square(e))) <= before
