@@ -761,10 +761,10 @@ int potential_system(nbr_ctx* c, double G, double eps2, double* dphi, size_t red
     double* sums = c->scr.red + red_off;
     int strips = 0;
     e = launch_energy((long long)s.n, eps2, ip, js, c->d_err, sums, c->sms, &strips, c->stream);
-    if (e == cudaSuccess) e = launch_rowsum(sums, strips, 1, sums + strips, c->stream);
+    if (e == cudaSuccess) e = launch_scaled_sum(sums, strips, kInvDistScale, sums + strips, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "energy launch");
     *dU = sums + strips;
-    *factor = -G * kInvDistScale;
+    *factor = -G;
     return NBR_OK;
   }
   *factor = 1.0;

@@ -331,6 +331,9 @@ cudaError_t launch_moments(long long n, long long n_pad, const double* x, const 
 // Sums nblocks rows of `width` doubles in block order (deterministic).
 cudaError_t launch_rowsum(const double* part, int nblocks, int width, double* out,
                           cudaStream_t stream);
+// *out = scale times the sum of n doubles in a fixed order.
+cudaError_t launch_scaled_sum(const double* part, int n, double scale, double* out,
+                              cudaStream_t stream);
 // Sets bit 0 of *flags if any x, y, z, (vx, vy, vz,) m entry is NaN or Inf,
 // bit 1 if a mass is negative (vx may be null: no velocities).
 cudaError_t launch_validate(long long n, const double* x, const double* y, const double* z,
