@@ -105,7 +105,9 @@ __device__ __forceinline__ void launch_dependents() {
 // Coordinates are relative to the tile's FP64 origin in FP32; per tile of 128
 // sources the FP32 action sums are added to FP64 sums.  The origin is the mean of
 // the tile's 128 particles, one of the first 32 counted twice: which one goes
-// with the row block.
+// with the row block.  It is taken from the tile's first particle, so that a
+// coordinate which all share is its origin exactly: the roundings of the mean of
+// 1e60 are past the range of FP32.
 //
 // Rounding: no more than in the kernels before (lane groups, tiles joined by
 // two_sum, reactions in FP64) takes two things.  With FINE a step's reaction
@@ -188,11 +190,14 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
       {
         const long long t0 = (long long)(b & ~3) * 32;
         const int left = (int)min(128LL, ip.n - t0);  // the tile's particles
+        const double fx = js.x[t0], fy = js.y[t0], fz = js.z[t0];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const int t = (lane + 32 * k) * left >> 7;
           const double w = k == 0 && lane == twice ? 2.0 : 1.0;
-          ox = fma(w, js.x[t0 + t], ox); oy = fma(w, js.y[t0 + t], oy); oz = fma(w, js.z[t0 + t], oz);
+          ox = fma(w, js.x[t0 + t] - fx, ox);
+          oy = fma(w, js.y[t0 + t] - fy, oy);
+          oz = fma(w, js.z[t0 + t] - fz, oz);
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
@@ -200,7 +205,7 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
           oy += __shfl_xor_sync(0xffffffffu, oy, off);
           oz += __shfl_xor_sync(0xffffffffu, oz, off);
         }
-        ox *= 1.0 / 129.0; oy *= 1.0 / 129.0; oz *= 1.0 / 129.0;
+        ox = fma(ox, 1.0 / 129.0, fx); oy = fma(oy, 1.0 / 129.0, fy); oz = fma(oz, 1.0 / 129.0, fz);
       }
       u64 XI[IP], YI[IP], ZI[IP], AX[IP], AY[IP], AZ[IP];
 #pragma unroll

@@ -89,6 +89,21 @@ def test_padding_of_the_last_batch(ctx, nbr, oracle, prec, n, case):
     check(ctx.forces(prec, eps2=eps2)[:, idx], ref, prec)
 
 
+# A coordinate that all particles share is as good as zero, however large
+@pytest.mark.parametrize("prec", [FP64, FP32C])
+@pytest.mark.parametrize("n", [4097, 4129, 8192])
+@pytest.mark.parametrize("far", [1e25, 1e60, 1e154, 1e300])
+def test_a_coordinate_all_share(ctx, nbr, prec, n, far):
+    s = {k: v.copy() for k, v in nbr.plummer(n, n).items() if k in "xyzm"}
+    a = []
+    for x in (0.0, far):
+        s["x"][:] = x
+        ctx.upload(s)
+        a.append(ctx.forces(prec, eps2=1e-4))
+    assert np.isfinite(a[0]).all()
+    np.testing.assert_array_equal(a[0], a[1])
+
+
 # two CTAs of the reduction per SM in all, and one batch more: 148 SMs, 296 batches
 @pytest.mark.parametrize("prec", [FP64, FP32C])
 @pytest.mark.parametrize("n", [9471, 9472, 9473, 9505])
