@@ -110,18 +110,19 @@ __device__ __forceinline__ void launch_dependents() {
 // 1e60 are past the range of FP32.
 //
 // Rounding: no more than in the kernels before (lane groups, tiles joined by
-// two_sum, reactions in FP64) takes two things.  With FINE a step's reaction
-// terms are added before they join the travelling sum, which is then a chain of
-// 32 additions instead of 16 NI.  And an origin of its own for each row block: a
-// source's coordinates are rounded anew for each, where with one origin all its
-// reactions carried the same displacement.  Median
-// error of a force (masses within a factor of three, eps 1e-3), before / one
-// chain and one origin / now: N = 6000 3.3e-8 / 4.2e-8 / 3.3e-8, 12001 3.7e-8 /
-// 4.7e-8 / 3.5e-8, 65536 3.6e-8 / 3.8e-8 / 3.1e-8, 262144 3.5e-8 / 3.5e-8 / 2.9e-8.
-// FINE costs 1 % at N = 12001 and 65536 (1364 -> 1384 us per evaluation) and 2.4 % at
-// 262144 (21.31 -> 21.83 ms); from kStripFine32 on the error is below the one
-// before without it (at 65536, one particle of a hundred 1000 times as heavy,
-// 4.8e-8 against 4.7e-8; at 131072 4.1e-8 against 4.2e-8).
+// two_sum, reactions in FP64) takes two things.  A reaction is no longer one chain
+// of 16 NI additions in each half: at NI = 16 it is added up in two parts of 16
+// steps, with a narrower block (FINE) a step's terms are added before they join
+// the travelling sum.  And an origin of its own for each row block: a source's
+// coordinates are rounded anew for each, where with one origin all its reactions
+// carried the same displacement.  Median error of a force (eps 1e-3), before / one
+// chain and one origin / now: masses within a factor of three N = 6000
+// 3.3e-8 / 4.1e-8 / 3.3e-8, 12001 3.8e-8 / 4.7e-8 / 3.6e-8, 65536 3.5e-8 / 3.7e-8 /
+// 3.0e-8, 262144 3.2e-8 / 3.1e-8 / 2.7e-8; masses over many decades (lognormal, one of
+// a hundred 1000 times as heavy) 14000 10.7e-8 / 10.1e-8 / 8.4e-8, 131073 6.5e-8 /
+// 7.5e-8 / 6.2e-8, 262143 6.0e-8 / 6.6e-8 / 5.2e-8.  FINE took 1.5 % more at NI = 16 than the parts (us per evaluation
+// 65536 1388 / 1371, 262144 21.76 / 21.48 ms; one chain 21.38), the parts 1.6 % more
+// than FINE at N = 8192 (32.7 / 32.2).
 //
 // The padding lanes of the last batch take the last particle's coordinates,
 // with their own mass, zero: the pair factor multiplies the masses last, and at
@@ -143,12 +144,13 @@ __device__ __forceinline__ double mass_mantissa(double m) {
                          : __hiloint2double((hi & 0x000fffff) | 0x3ff00000, __double2loint(m));
 }
 
-constexpr long long kStripFine32 = 1LL << 17;
-template <int NI, bool EXCL, bool FINE>
+template <int NI, bool EXCL>
 __global__ void __launch_bounds__(kStripWarps * 32, 1)
     k_strip_f32c(const IParticles ip, const JStream js, const StripPlan sp, const float eps2f,
                  double* act, float* rea, int* err) {
   constexpr int IP = NI / 2, TB = NI;
+  constexpr bool FINE = NI < 16;
+  constexpr int PART = FINE ? 32 : 16;  // steps of a reaction's chain
   extern __shared__ double strip_acc[];  // [kStripWarps][3][32 NI]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = warp * gridDim.x + blockIdx.x;
@@ -158,7 +160,7 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
   if (g >= sp.strips) return;
   int u = strip_start(sp, g);
   const int u_end = strip_start(sp, g + 1);
-  const int from = (lane + 31) & 31;
+  const int from = (lane + 31) & 31, from_part = (lane + 32 - PART) & 31;
   const u64 EPS2 = pack2(eps2f, eps2f), C53 = pack2(kC53, kC53);
   double* acc = strip_acc + warp * (96 * NI) + lane;
   for (int r = strip_row(sp, u); u < u_end; ++r) {
@@ -221,66 +223,71 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
         const long long j = 32LL * b + lane, jx = min(j, ip.n - 1);
         float sx = __double2float_rn(js.x[jx] - ox), sy = __double2float_rn(js.y[jx] - oy),
               sz = __double2float_rn(js.z[jx] - oz), sm = (float)(unit * js.m[j]);
-        u64 RX = 0ull, RY = 0ull, RZ = 0ull;
+        float qx = 0.f, qy = 0.f, qz = 0.f;  // the reaction of the parts before
+#pragma unroll 1
+        for (int part = 0; part < 32 / PART; ++part) {
+          u64 RX = 0ull, RY = 0ull, RZ = 0ull;
 #pragma unroll(NI >= 12 ? 2 : 4)
-        for (int step = 0; step < 32; ++step) {
-          const u64 SX = pack2(sx, sx), SY = pack2(sy, sy), SZ = pack2(sz, sz), SM = pack2(sm, sm);
-          u64 dx[IP], dy[IP], dz[IP], r2[IP], y[IP], y2[IP], c[IP];
+          for (int step = 0; step < PART; ++step) {
+            const u64 SX = pack2(sx, sx), SY = pack2(sy, sy), SZ = pack2(sz, sz), SM = pack2(sm, sm);
+            u64 dx[IP], dy[IP], dz[IP], r2[IP], y[IP], y2[IP], c[IP];
 #pragma unroll
-          for (int p = 0; p < IP; ++p) dx[p] = sub2(SX, XI[p]);
+            for (int p = 0; p < IP; ++p) dx[p] = sub2(SX, XI[p]);
 #pragma unroll
-          for (int p = 0; p < IP; ++p) dy[p] = sub2(SY, YI[p]);
+            for (int p = 0; p < IP; ++p) dy[p] = sub2(SY, YI[p]);
 #pragma unroll
-          for (int p = 0; p < IP; ++p) dz[p] = sub2(SZ, ZI[p]);
+            for (int p = 0; p < IP; ++p) dz[p] = sub2(SZ, ZI[p]);
 #pragma unroll
-          for (int p = 0; p < IP; ++p) r2[p] = fma2(dx[p], dx[p], EPS2);
+            for (int p = 0; p < IP; ++p) r2[p] = fma2(dx[p], dx[p], EPS2);
 #pragma unroll
-          for (int p = 0; p < IP; ++p) r2[p] = fma2(dy[p], dy[p], r2[p]);
+            for (int p = 0; p < IP; ++p) r2[p] = fma2(dy[p], dy[p], r2[p]);
 #pragma unroll
-          for (int p = 0; p < IP; ++p) r2[p] = fma2(dz[p], dz[p], r2[p]);
+            for (int p = 0; p < IP; ++p) r2[p] = fma2(dz[p], dz[p], r2[p]);
 #pragma unroll
-          for (int p = 0; p < IP; ++p) {
-            if (EXCL) {
-              float rl, rh;
-              unpack2(r2[p], rl, rh);
-              y[p] = pack2(rl > 0.f ? rsqrt_mufu(rl) : 0.f, rh > 0.f ? rsqrt_mufu(rh) : 0.f);
-            } else {
-              y[p] = rsqrt2(r2[p]);
+            for (int p = 0; p < IP; ++p) {
+              if (EXCL) {
+                float rl, rh;
+                unpack2(r2[p], rl, rh);
+                y[p] = pack2(rl > 0.f ? rsqrt_mufu(rl) : 0.f, rh > 0.f ? rsqrt_mufu(rh) : 0.f);
+              } else {
+                y[p] = rsqrt2(r2[p]);
+              }
             }
+#pragma unroll
+            for (int p = 0; p < IP; ++p) y2[p] = mul2(y[p], y[p]);
+#pragma unroll
+            for (int p = 0; p < IP; ++p) c[p] = fnma2(r2[p], y2[p], C53);
+#pragma unroll
+            for (int p = 0; p < IP; ++p) y2[p] = mul2(y2[p], y[p]);
+#pragma unroll
+            for (int p = 0; p < IP; ++p) c[p] = mul2(y2[p], c[p]);
+            u64 tx = RX, ty = RY, tz = RZ;  // FINE: the step's reaction alone
+#pragma unroll
+            for (int p = 0; p < IP; ++p) {
+              const u64 sj = mul2(c[p], SM), si = mul2(c[p], MI[p]);
+              tx = FINE && p == 0 ? mul2(si, dx[p]) : fma2(si, dx[p], tx);
+              ty = FINE && p == 0 ? mul2(si, dy[p]) : fma2(si, dy[p], ty);
+              tz = FINE && p == 0 ? mul2(si, dz[p]) : fma2(si, dz[p], tz);
+              AZ[p] = fma2(sj, dz[p], AZ[p]);
+              AY[p] = fma2(sj, dy[p], AY[p]);
+              AX[p] = fma2(sj, dx[p], AX[p]);
+            }
+            RX = __shfl_sync(0xffffffffu, FINE ? add2(RX, tx) : tx, from);
+            RY = __shfl_sync(0xffffffffu, FINE ? add2(RY, ty) : ty, from);
+            RZ = __shfl_sync(0xffffffffu, FINE ? add2(RZ, tz) : tz, from);
+            sx = __shfl_sync(0xffffffffu, sx, from);
+            sy = __shfl_sync(0xffffffffu, sy, from);
+            sz = __shfl_sync(0xffffffffu, sz, from);
+            sm = __shfl_sync(0xffffffffu, sm, from);
           }
-#pragma unroll
-          for (int p = 0; p < IP; ++p) y2[p] = mul2(y[p], y[p]);
-#pragma unroll
-          for (int p = 0; p < IP; ++p) c[p] = fnma2(r2[p], y2[p], C53);
-#pragma unroll
-          for (int p = 0; p < IP; ++p) y2[p] = mul2(y2[p], y[p]);
-#pragma unroll
-          for (int p = 0; p < IP; ++p) c[p] = mul2(y2[p], c[p]);
-          u64 tx = RX, ty = RY, tz = RZ;  // FINE: the step's reaction alone
-#pragma unroll
-          for (int p = 0; p < IP; ++p) {
-            const u64 sj = mul2(c[p], SM), si = mul2(c[p], MI[p]);
-            tx = FINE && p == 0 ? mul2(si, dx[p]) : fma2(si, dx[p], tx);
-            ty = FINE && p == 0 ? mul2(si, dy[p]) : fma2(si, dy[p], ty);
-            tz = FINE && p == 0 ? mul2(si, dz[p]) : fma2(si, dz[p], tz);
-            AZ[p] = fma2(sj, dz[p], AZ[p]);
-            AY[p] = fma2(sj, dy[p], AY[p]);
-            AX[p] = fma2(sj, dx[p], AX[p]);
-          }
-          RX = __shfl_sync(0xffffffffu, FINE ? add2(RX, tx) : tx, from);
-          RY = __shfl_sync(0xffffffffu, FINE ? add2(RY, ty) : ty, from);
-          RZ = __shfl_sync(0xffffffffu, FINE ? add2(RZ, tz) : tz, from);
-          sx = __shfl_sync(0xffffffffu, sx, from);
-          sy = __shfl_sync(0xffffffffu, sy, from);
-          sz = __shfl_sync(0xffffffffu, sz, from);
-          sm = __shfl_sync(0xffffffffu, sm, from);
+          float l, h;
+          unpack2(RX, l, h); qx = __shfl_sync(0xffffffffu, qx, from_part) + (l + h);
+          unpack2(RY, l, h); qy = __shfl_sync(0xffffffffu, qy, from_part) + (l + h);
+          unpack2(RZ, l, h); qz = __shfl_sync(0xffffffffu, qz, from_part) + (l + h);
         }
         if (b >= b_rea) {
           float* o = out + 96LL * b;
-          float l, h;
-          unpack2(RX, l, h); o[0] = -(l + h);
-          unpack2(RY, l, h); o[32] = -(l + h);
-          unpack2(RZ, l, h); o[64] = -(l + h);
+          o[0] = -qx; o[32] = -qy; o[64] = -qz;
         }
       }
 #pragma unroll
@@ -698,25 +705,22 @@ std::vector<int> strip_bands(int precision, long long n, int sms, int ni, int ba
 
 namespace {
 
-template <int NI, bool FINE>
+template <int NI>
 const void* strip_f32c(bool excl) {
-  return excl ? (const void*)k_strip_f32c<NI, true, FINE> : (const void*)k_strip_f32c<NI, false, FINE>;
+  return excl ? (const void*)k_strip_f32c<NI, true> : (const void*)k_strip_f32c<NI, false>;
 }
-template <int NI, bool FINE>
-const void* strip_f64(bool excl) {
-  return excl ? (const void*)k_strip_f64<NI, true, FINE> : (const void*)k_strip_f64<NI, false, FINE>;
-}
-template <bool FINE>
-const void* strip_fn(int precision, int ni, bool excl) {
-  if (precision == kFP32C)
-    return ni == 8 ? strip_f32c<8, FINE>(excl) : ni == 10 ? strip_f32c<10, FINE>(excl)
-                                               : ni == 16 ? strip_f32c<16, FINE>(excl) : nullptr;
-  return ni == 6 ? strip_f64<6, FINE>(excl) : ni == 8 ? strip_f64<8, FINE>(excl)
-                                            : ni == 10 ? strip_f64<10, FINE>(excl) : nullptr;
+template <int NI>
+const void* strip_f64(bool excl, bool fine) {
+  if (fine) return excl ? (const void*)k_strip_f64<NI, true, true> : (const void*)k_strip_f64<NI, false, true>;
+  return excl ? (const void*)k_strip_f64<NI, true, false> : (const void*)k_strip_f64<NI, false, false>;
 }
 const void* strip_fn(int precision, int ni, bool excl, long long n) {
-  return n < (precision == kFP32C ? kStripFine32 : kStripFine64) ? strip_fn<true>(precision, ni, excl)
-                                                                 : strip_fn<false>(precision, ni, excl);
+  if (precision == kFP32C)
+    return ni == 8 ? strip_f32c<8>(excl) : ni == 10 ? strip_f32c<10>(excl)
+                                         : ni == 16 ? strip_f32c<16>(excl) : nullptr;
+  const bool fine = n < kStripFine64;
+  return ni == 6 ? strip_f64<6>(excl, fine) : ni == 8 ? strip_f64<8>(excl, fine)
+                                            : ni == 10 ? strip_f64<10>(excl, fine) : nullptr;
 }
 
 // The action sums of every warp's row block.

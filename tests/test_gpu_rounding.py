@@ -66,6 +66,18 @@ def test_fp32c_strips(ctx, nbr, oracle, n, other, eps2):
     assert strips <= 1.1 * before, (strips, before)
 
 
+# Masses over many decades, one of a hundred bodies 1000 times as heavy: median errors
+# of the CTA grid, which served these sizes; with one chain of additions per
+# reaction the strips had 8.1e-8 and 8.3e-8
+@pytest.mark.parametrize("n,before", [(131073, 7.30e-8), (200000, 7.33e-8)])
+def test_fp32c_strips_masses_over_decades(ctx, nbr, oracle, n, before):
+    s, g = nbr.plummer(n, n + 1), np.random.default_rng(n)
+    s["m"] = g.lognormal(0.0, 2.0, n) * np.where(g.uniform(size=n) < 0.01, 1000.0, 1.0)
+    s["m"] /= s["m"].sum()
+    strips, = median_errors(ctx, oracle, s, FP32C, 1e-6, [(3, 8)])
+    assert strips <= before
+
+
 # Masses in whole ratios carry no rounding of their own: a system whose masses are
 # multiples of 1/7000 moves as one of multiples of 2^-13 (exact in 32 bits), up to
 # the roundings of the factor, the sums' product with it and this quotient

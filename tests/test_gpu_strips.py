@@ -170,7 +170,8 @@ def test_energy_of_an_extreme_pair(ctx, d):
     assert ctx.diagnostics()["U"] == 0.0 and ctx.potential(per_particle=True)[0] == 0.0
 
 
-# Where the reactions' form changes (FP64 12288, FP32C 131072 particles), ragged too
+# Where the FP64 reactions' form changes (12288 particles), and a large FP32C system,
+# ragged too
 @pytest.mark.parametrize("prec,n", [(FP64, 12287), (FP64, 12288), (FP64, 12289),
                                     (FP32C, 131071), (FP32C, 131072), (FP32C, 131073)])
 @pytest.mark.parametrize("eps2", [0.0, 1e-6])
