@@ -317,13 +317,16 @@ __global__ void __launch_bounds__(kStripWarps * 32, 1)
 // large below 10000 particles.  So every 128 sources the action sums go to a
 // second level in shared memory (no cost measured), with FINE a step's
 // NI reaction terms are added before they join the travelling sum (three more
-// adds per step, 2 % of the time; taken below kStripFine64, above it the sums
-// are more exact than before without it), and the reduction adds its warps' sums
-// by halves (in order their last roundings alone made half of the error).
-// Median error of a force, eps = 0 .. 1e-2, the kernel before / now: N = 4200 1.05e-16 /
-// 0.86e-16, 9000 1.16e-16 / 0.84e-16, 14000 1.03e-16 / 0.92e-16, 32768 2.0e-16 /
-// 0.88e-16.
-constexpr long long kStripFine64 = 12288;
+// adds per step, 1.3 % of the time; taken below kStripFine64, from where the kernel
+// before was the CTA grid and the sums are more exact without it), and the
+// reduction adds its warps' sums by halves (in order their last roundings alone
+// made half of the error).  Median error of a force (eps 1e-3), the kernel before / in
+// one chain, the sums in order / now: N = 4200 1.24e-16 / 1.37e-16 / 1.02e-16, 9000
+// 1.31e-16 / 1.32e-16 / 1.00e-16, 14000 1.18e-16 / 1.33e-16 / 0.98e-16 (1.07e-16 without
+// FINE), 65536 3.9e-16 / 1.4e-16 / 1.1e-16; masses over many decades (lognormal, one of a
+// hundred 1000 times as heavy) 14000 1.83e-16 / 2.1e-16 / 1.47e-16 (1.83e-16 without; at
+// eps 1e-2 1.81e-16, 1.92e-16 without).
+constexpr long long kStripFine64 = 16384;
 template <int NI, bool EXCL, bool FINE>
 __global__ void __launch_bounds__(kStripWarps * 32, 1)
     k_strip_f64(const IParticles ip, const JStream js, const StripPlan sp, const double eps2,

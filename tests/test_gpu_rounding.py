@@ -18,6 +18,14 @@ def system(nbr, n, masses):
     return s
 
 
+def over_decades(nbr, n):
+    """Masses over many decades, one of a hundred 1000 times as heavy."""
+    s, g = nbr.plummer(n, n + 1), np.random.default_rng(n)
+    s["m"] = g.lognormal(0.0, 2.0, n) * np.where(g.uniform(size=n) < 0.01, 1000.0, 1.0)
+    s["m"] /= s["m"].sum()
+    return s
+
+
 def median_errors(ctx, oracle, s, prec, eps2, configs):
     """One median per (ni, warps); "run": the accelerations of a run's kernel, as
     the velocities after one Euler step of size 1 from rest."""
@@ -49,6 +57,14 @@ def test_fp64_strips(ctx, nbr, oracle, n, eps2):
     assert strips <= 1.03 * small, (strips, small)
 
 
+# and with masses over many decades
+@pytest.mark.parametrize("n", [12288, 14000])
+@pytest.mark.parametrize("eps2", [0.0, 1e-4])
+def test_fp64_strips_masses_over_decades(ctx, nbr, oracle, n, eps2):
+    strips, small = median_errors(ctx, oracle, over_decades(nbr, n), FP64, eps2, [(3, 8), (1, 8)])
+    assert strips <= 1.03 * small, (strips, small)
+
+
 # the persistent run against the force call of the same size
 @pytest.mark.parametrize("n", [1000, 2048, 4096])
 def test_fp64_persistent_run(ctx, nbr, oracle, n):
@@ -66,15 +82,11 @@ def test_fp32c_strips(ctx, nbr, oracle, n, other, eps2):
     assert strips <= 1.1 * before, (strips, before)
 
 
-# Masses over many decades, one of a hundred bodies 1000 times as heavy: median errors
-# of the CTA grid, which served these sizes; with one chain of additions per
-# reaction the strips had 8.1e-8 and 8.3e-8
+# Median errors of the CTA grid, which served these sizes; with one chain of additions
+# per reaction the strips had 8.1e-8 and 8.3e-8
 @pytest.mark.parametrize("n,before", [(131073, 7.30e-8), (200000, 7.33e-8)])
 def test_fp32c_strips_masses_over_decades(ctx, nbr, oracle, n, before):
-    s, g = nbr.plummer(n, n + 1), np.random.default_rng(n)
-    s["m"] = g.lognormal(0.0, 2.0, n) * np.where(g.uniform(size=n) < 0.01, 1000.0, 1.0)
-    s["m"] /= s["m"].sum()
-    strips, = median_errors(ctx, oracle, s, FP32C, 1e-6, [(3, 8)])
+    strips, = median_errors(ctx, oracle, over_decades(nbr, n), FP32C, 1e-6, [(3, 8)])
     assert strips <= before
 
 

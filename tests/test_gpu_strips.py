@@ -170,9 +170,9 @@ def test_energy_of_an_extreme_pair(ctx, d):
     assert ctx.diagnostics()["U"] == 0.0 and ctx.potential(per_particle=True)[0] == 0.0
 
 
-# Where the FP64 reactions' form changes (12288 particles), and a large FP32C system,
+# Where the FP64 reactions' form changes (16384 particles), and a large FP32C system,
 # ragged too
-@pytest.mark.parametrize("prec,n", [(FP64, 12287), (FP64, 12288), (FP64, 12289),
+@pytest.mark.parametrize("prec,n", [(FP64, 16383), (FP64, 16384), (FP64, 16385),
                                     (FP32C, 131071), (FP32C, 131072), (FP32C, 131073)])
 @pytest.mark.parametrize("eps2", [0.0, 1e-6])
 def test_reactions_where_their_form_changes(ctx, nbr, oracle, prec, n, eps2):
